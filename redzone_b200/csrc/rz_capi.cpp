@@ -391,7 +391,7 @@ int rz_keep(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, const uin
     if (st != RZ_OK) return st;
     st = launch_keep(ctx, d_data, uint32_t(n), elem_bytes, d_keep, uint32_t(m), ctx->ws.keep_stage, s);
     if (st != RZ_OK) return st;
-    ctx->last_kernels = m > 0 ? 1 : 0;
+    ctx->last_kernels = m > 0 ? 2 : 0;
     if (flags & RZ_SYNC) return read_status(ctx, s);
     return RZ_OK;
 }

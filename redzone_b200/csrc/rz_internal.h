@@ -136,7 +136,7 @@ constexpr uint32_t kClusterMaxK = 1u << 14;  // RZ_SCHED_AUTO uses the cluster s
 constexpr int kConfigSpace = 63;
 void config_space(rz_launch_cfg* out);
 int launch_validate(rz_ctx* ctx, uint32_t n, const uint32_t* idx, uint32_t k, cudaStream_t s);
-// rz_keep: gather data[keep[j]] into `stage` (m items), then copy the stage to data[0..m).
+// rz_keep: data[0..m) = old data[keep[j]] in two kernels; `stage` holds m items (those kept from [0, m)).
 int launch_keep(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* keep, uint32_t m, void* stage,
                 cudaStream_t s);
 // Largest block size the single-list kernel for (w, items) can launch with.

@@ -1,0 +1,48 @@
+"""GPU tests of kernels at the edges of their tiles and dispatch rules, bit-exact against the
+oracle or a plain numpy statement of the same result."""
+import numpy as np
+import pytest
+import torch
+
+import redzone_b200 as rz
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = rz.Context(0)
+    yield c
+    c.close()
+
+
+def payload(n: int, words: int, seed: int) -> np.ndarray:
+    return np.random.default_rng(seed).integers(0, 1 << 32, size=(n, words), dtype=np.uint64).astype(np.uint32)
+
+
+def on_gpu(a: np.ndarray):
+    return torch.from_numpy(a.view(np.int32).copy()).to(DEV)
+
+
+@pytest.mark.parametrize("words", [1, 2, 4, 8])
+@pytest.mark.parametrize("m", [1, 255, 1023, 1024, 1025, 5000])
+def test_keep_in_two_kernels(ctx, words, m):
+    """rz_keep around one 1024-item block: entries on both sides of m (items kept from [0, m) go
+    through the scratch), the same row several times, one entry past the end."""
+    n = 5001
+    rng = np.random.default_rng(m * 8 + words)
+    host = payload(n, words, seed=m)
+    keep = rng.integers(0, n, size=m).astype(np.uint32)
+    keep[:: 3] = rng.integers(0, m, size=keep[:: 3].size)
+    d = on_gpu(host)
+    assert ctx.keep(d, on_gpu(keep), flags=rz.RZ_SYNC) == m
+    got = d.cpu().numpy().view(np.uint32)
+    assert np.array_equal(got[:m], host[keep]) and np.array_equal(got[m:], host[m:])
+    keep[m // 2] = n
+    d = on_gpu(host)
+    with pytest.raises(rz.RedzoneError):
+        ctx.keep(d, on_gpu(keep), flags=rz.RZ_SYNC)
+    exp = host[np.minimum(keep, n - 1)]
+    exp[m // 2] = host[m // 2]
+    assert np.array_equal(d.cpu().numpy().view(np.uint32)[:m], exp)
