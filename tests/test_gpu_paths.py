@@ -46,3 +46,29 @@ def test_keep_in_two_kernels(ctx, words, m):
     exp = host[np.minimum(keep, n - 1)]
     exp[m // 2] = host[m // 2]
     assert np.array_equal(d.cpu().numpy().view(np.uint32)[:m], exp)
+
+
+@pytest.mark.parametrize("n,k,place", [(511, 40, "spread"), (512, 512, "spread"), (513, 1, "end"), (70001, 3000, "spread"),
+                                       (1 << 20, 60000, "run"), ((1 << 20) + 77, 60000, "run"), (4099, 0, "spread")])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_produced_rows_of_the_key_filter(ctx, n, k, place, shift):
+    """rz_produce_where_less emits exactly the rows below the threshold: around one warp step (512
+    keys), runs long enough that blocks collect more rows than their buffer holds, keys off the
+    16-byte boundary (shift), and the removal agrees with rz_remove on the list it wrote."""
+    rng = np.random.default_rng(n + k)
+    rows = {"spread": lambda: rng.choice(n, size=k, replace=False), "run": lambda: np.arange(n // 3, n // 3 + k),
+            "end": lambda: np.arange(n - k, n)}[place]()
+    keys = np.full(n + shift, 900, np.uint32)
+    keys[shift + rows] = 100
+    d_keys = on_gpu(keys)[shift:]
+    p = rz.Producer(ctx, capacity=max(1, k + 5))
+    p.reset(n)
+    p.produce_where_less(d_keys, 500)
+    lst, kk, _ = p.download()
+    assert kk == k and np.array_equal(np.sort(lst), np.sort(rows).astype(np.uint32))
+    host = payload(n, 1, seed=n)
+    a, b = on_gpu(host), on_gpu(host)
+    assert p.remove(a, flags=rz.RZ_SYNC) == n - k
+    if k:
+        ctx.remove(b, on_gpu(lst), flags=rz.RZ_SYNC)
+    assert torch.equal(a, b)
