@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+import oracle
 import redzone_b200 as rz
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +73,38 @@ def test_produced_rows_of_the_key_filter(ctx, n, k, place, shift):
     if k:
         ctx.remove(b, on_gpu(lst), flags=rz.RZ_SYNC)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 4097, 100003])
+@pytest.mark.parametrize("share", [2, 255, 257, 4000])
+def test_validation_both_ways(ctx, n, share):
+    """RZ_VALIDATE with lists long and short for their n (map zeroed as a whole / entry by entry): a
+    valid list passes, also after one with a duplicate or an entry past the end (or both), which is
+    reported and moves nothing."""
+    k = max(1, n // share)
+    rng = np.random.default_rng(n + share)
+    host = payload(n, 1, seed=n)
+    good = rng.choice(n, size=k, replace=False).astype(np.uint32)
+    bad = []
+    if k > 1:
+        dup = good.copy()
+        dup[-1] = dup[0]
+        bad.append((dup, 2))
+    out = good.copy()
+    out[k // 2] = n
+    bad.append((out, 3))
+    if k > 2:
+        both = out.copy()
+        both[0] = both[k - 1]
+        bad.append((both, 3))
+    for idx, code in bad:
+        d = on_gpu(host)
+        with pytest.raises(rz.RedzoneError) as e:
+            ctx.remove(d, on_gpu(idx), flags=rz.RZ_VALIDATE | rz.RZ_SYNC)
+        assert e.value.code == code
+        assert np.array_equal(d.cpu().numpy().view(np.uint32), host)
+        d = on_gpu(host)
+        assert ctx.remove(d, on_gpu(good), flags=rz.RZ_VALIDATE | rz.RZ_SYNC) == n - k
+        exp = host.copy()
+        oracle.remove(exp, good)
+        assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n - k], exp[: n - k])
