@@ -72,10 +72,10 @@ int ensure_seen(rz_ctx* ctx, size_t n) {
 int ensure_partition(rz_ctx* ctx, size_t n, size_t ntiles) {
     int st = grow(ctx, ctx->ws.part_bits, ctx->ws.part_words, (n + 31) / 32 + 1, true);
     if (st != RZ_OK) return st;
-    // Ticket line (16 words), three 32-bit arrays of ntiles rounded up to 4 (staged, kept,
-    // offset), then one 16-byte record per tile.
+    // Ticket line (16 words), two 32-bit arrays of ntiles rounded up to 4 (staged, offset), one
+    // 16-byte record per tile, then one and a total for each of at most 2048 runs of tiles.
     const size_t ntp = (ntiles + 3) & ~size_t(3);
-    return grow(ctx, ctx->ws.tile_state, ctx->ws.tile_cap, 16 + 3 * ntp / 2 + 2 * ntiles + 1, true);
+    return grow(ctx, ctx->ws.tile_state, ctx->ws.tile_cap, 16 + ntp + 2 * ntiles + 2 * 2048 + 1024, true);
 }
 
 int reset_if_dirty(rz_ctx* ctx, cudaStream_t s) {
@@ -84,6 +84,7 @@ int reset_if_dirty(rz_ctx* ctx, cudaStream_t s) {
     if (w.bitmap) RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.bitmap, 0, w.bitmap_words * 4, s));
     if (w.seen) RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.seen, 0, w.seen_words * 4, s));
     if (w.part_bits) RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.part_bits, 0, w.part_words * 4, s));
+    if (w.tile_state) RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.tile_state, 0, 128, s));
     RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.epoch, 0, 4, s));
     RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.split_count, 0, 8, s));
     RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.arrive, 0, kMaxGrid * 4, s));

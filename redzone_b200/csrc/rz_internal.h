@@ -39,7 +39,7 @@ struct Workspace {
     size_t seen_words = 0;
     uint32_t* part_bits = nullptr;   // partition path: n-bit removal map
     size_t part_words = 0;
-    unsigned long long* tile_state = nullptr;  // partition path: ticket, staged/kept/offset per tile
+    unsigned long long* tile_state = nullptr;  // partition path: ticket, staged / offset / record per tile
     size_t tile_cap = 0;
     unsigned long long* dev_len = nullptr;     // device copy of the last new length
     uint32_t* idx_stage = nullptr;   // rz_remove_host_idx: device copy of host indices

@@ -5,10 +5,11 @@
 // out of place) or thrust::remove (Thrust_remove.hxx:15-17, in place). Here the same three steps
 // run in place on B200:
 //   1. mark:  the k removed positions set bits of an n-bit map in scratch (any payload width);
-//   2. count: kept items per tile from the bit map alone (n/8 bytes), then one CTA turns the
-//             per-tile counts into exclusive output offsets;
+//   2. count: kept items per tile from the bit map alone (n/8 bytes); every block turns the counts of
+//             its run of tiles into offsets inside the run, the last block the runs' totals into
+//             their offsets;
 //   3. move:  each tile stages its kept items in shared memory, raises its "staged" flag, and
-//             writes them to offset[t] + rank.
+//             writes them to (offset of the run) + (offset in it) + rank.
 // In-place safety without a chained look-back: tile t writes [offset[t], offset[t] + kept[t]),
 // a range shorter than one tile that ends at or before the end of tile t's own input, so it
 // overlaps the input of at most two tiles u <= t; tile t waits only for those tiles' staged flags.
@@ -25,123 +26,118 @@ namespace rz {
 
 constexpr int kPartBlock = 512;
 
-__global__ void partition_mark_kernel(const uint32_t* __restrict__ idx, uint32_t k, uint32_t n,
-                                      uint32_t* __restrict__ bits, uint32_t* status, uint32_t validate) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) {
-        const uint32_t r = __ldg(&idx[i]);
-        if (r >= n) {
-            atomicOr(status, ST_RANGE);
-            continue;
+// Bound by the map's atomics (1.75e11 per second): kPartMarkLoads entries in flight per thread, and no
+// result asked for unless the list is validated. 10M entries of n = 100M: 58 us, 89 with one entry at
+// a time and the old word always asked for.
+constexpr int kPartMarkLoads = 8;
+template <bool VALIDATE>
+__global__ void __launch_bounds__(256) partition_mark_kernel(const uint32_t* __restrict__ idx, uint32_t k, uint32_t n,
+                                                             uint32_t* __restrict__ bits, uint32_t* status) {
+    const uint64_t stride = uint64_t(gridDim.x) * 256 * kPartMarkLoads;
+    uint32_t found = 0;
+    for (uint64_t b = uint64_t(blockIdx.x) * (256 * kPartMarkLoads) + threadIdx.x; b < k; b += stride) {
+        uint32_t r[kPartMarkLoads];
+#pragma unroll
+        for (int j = 0; j < kPartMarkLoads; ++j) {
+            const uint64_t i = b + uint64_t(j) * 256;
+            r[j] = i < k ? __ldg(&idx[i]) : 0u;
         }
-        const uint32_t bit = 1u << (r & 31u);
-        const uint32_t old = atomicOr(&bits[r >> 5], bit);
-        if (validate && (old & bit)) atomicOr(status, ST_DUPLICATE);
+#pragma unroll
+        for (int j = 0; j < kPartMarkLoads; ++j) {
+            if (b + uint64_t(j) * 256 >= k) continue;
+            const uint32_t bit = 1u << (r[j] & 31u);
+            if (r[j] >= n) found |= ST_RANGE;
+            else if (!VALIDATE) atomicOr(&bits[r[j] >> 5], bit);
+            else if (atomicOr(&bits[r[j] >> 5], bit) & bit) found |= ST_DUPLICATE;
+        }
     }
+    if (found) atomicOr(status, found);
 }
 
-// Kept items of each tile (one warp per tile, grid-stride over tiles). The bit map is padded with
-// zero words to whole tiles, so every tile's BW words are read as BW/4 16-byte loads, all issued
-// before any is used; only bits past n are masked.
+// Kept items of each tile, one warp per tile, each block a run of `run` consecutive tiles: per tile
+// the record {kept items of the run before it, kept items, 0, 0} that the pipelined move copies with
+// the tile (and the offset alone for the other move), per run one {kept items before the run, 0, 0, 0},
+// made by the last block from the runs' totals. Also clears the move's ticket and staged flags, so that
+// the call needs no memset and stays correct when it is replayed from a CUDA graph. The bit map is
+// padded with zero words to whole tiles, so every tile's BW words are read as BW/4 16-byte loads,
+// all issued before any is used; only bits past n are masked.
+// 12208 tiles: 9.8 us; counts, then a scan of all tiles by one block: 5 + 10 us, and a memset before.
+constexpr uint32_t kPartMaxRun = 4096, kPartMaxRuns = 2048;
+struct PartScratch {
+    unsigned long long* ticket;  // its own 128-byte line; [1]: blocks of the count kernel done (left zero)
+    uint32_t* staged;            // per tile
+    uint32_t* offset;            // per tile
+    uint4* recs;                 // per tile
+    uint4* run_recs;             // per run
+    uint32_t* run_total;         // per run
+};
 template <uint32_t BW>
-__global__ void partition_count_kernel(const uint32_t* __restrict__ bits, uint32_t n, uint32_t ntiles,
-                                       uint32_t* __restrict__ kept) {
+__global__ void __launch_bounds__(256) partition_count_kernel(const uint32_t* __restrict__ bits, uint32_t n,
+                                                              uint32_t ntiles, uint32_t run, const PartScratch p) {
     constexpr uint32_t TILE = BW * 32u;
     constexpr int V = int((BW / 4 + 31) / 32);  // 16-byte loads per lane
+    __shared__ uint32_t s_kept[kPartMaxRun + 1];
+    __shared__ uint32_t s_scan[33];
+    __shared__ uint32_t s_last;
     const int lane = threadIdx.x & 31;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntiles; t += warps) {
+    const uint32_t t0 = blockIdx.x * run, m = min(run, ntiles - t0);
+    for (uint32_t q = threadIdx.x >> 5; q < m; q += 8) {
+        const uint32_t t = t0 + q;
         const uint4* src = reinterpret_cast<const uint4*>(bits + size_t(t) * BW);
         uint4 v[V];
 #pragma unroll
         for (int j = 0; j < V; ++j) {
-            const uint32_t q = uint32_t(j) * 32u + uint32_t(lane);
-            v[j] = q < BW / 4 ? __ldg(&src[q]) : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t u = uint32_t(j) * 32u + uint32_t(lane);
+            v[j] = u < BW / 4 ? __ldg(&src[u]) : make_uint4(0u, 0u, 0u, 0u);
         }
         uint32_t removed = 0;
 #pragma unroll
         for (int j = 0; j < V; ++j) {
-            const uint32_t q = uint32_t(j) * 32u + uint32_t(lane);
+            const uint32_t u = uint32_t(j) * 32u + uint32_t(lane);
             const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const uint32_t first = t * TILE + (q * 4u + uint32_t(e)) * 32u;
+                const uint64_t first = uint64_t(t) * TILE + (u * 4u + uint32_t(e)) * 32u;
                 uint32_t word = w[e];
                 if (first >= n) word = 0u;
                 else if (n - first < 32u) word &= (1u << (n - first)) - 1u;  // bits past n are not items
                 removed += __popc(word);
             }
         }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) removed += __shfl_down_sync(0xffffffffu, removed, d);
-        if (lane == 0) kept[t] = min(TILE, n - t * TILE) - removed;
+        removed = __reduce_add_sync(0xffffffffu, removed);
+        if (lane == 0) s_kept[q] = uint32_t(min(uint64_t(TILE), uint64_t(n) - uint64_t(t) * TILE)) - removed;
     }
-}
-
-// Exclusive scan of kept[0..ntiles) into offset[0..ntiles) and the per-tile records
-// {offset, kept, 0, 0} the pipelined move copies with each tile; one CTA of 1024 threads.
-// Chunks of kScanChunk counts are loaded coalesced (all loads in flight at once) into shared
-// memory, each thread sums a contiguous run of 32, one block scan, and the results are written
-// back coalesced; a running carry joins the chunks.
-constexpr uint32_t kScanChunk = 32768;
-// One padding word per 32 keeps both the coalesced and the per-thread-run accesses free of bank
-// conflicts.
-__device__ __forceinline__ uint32_t scan_pad(uint32_t i) { return i + (i >> 5); }
-constexpr size_t kScanSmem = size_t(kScanChunk + kScanChunk / 32) * 4;
-__global__ void __launch_bounds__(1024) partition_scan_kernel(const uint32_t* __restrict__ kept, uint32_t ntiles,
-                                                              uint32_t* __restrict__ offset, uint4* __restrict__ recs) {
-    extern __shared__ uint32_t s_kept[];  // [kScanChunk + kScanChunk / 32], padded
-    __shared__ uint32_t scratch[33];
-    constexpr uint32_t B = 1024, PER = kScanChunk / B;
-    uint32_t carry = 0;
-    for (uint32_t c0 = 0; c0 < ntiles; c0 += kScanChunk) {
-        const uint32_t cn = min(kScanChunk, ntiles - c0);
-        {
-            uint32_t v[PER];
-#pragma unroll
-            for (uint32_t j = 0; j < PER; ++j) {
-                const uint32_t q = j * B + threadIdx.x;
-                v[j] = q < cn ? kept[c0 + q] : 0u;
-            }
-#pragma unroll
-            for (uint32_t j = 0; j < PER; ++j) s_kept[scan_pad(j * B + threadIdx.x)] = v[j];
-        }
-        __syncthreads();
-        uint32_t s = 0;
-#pragma unroll
-        for (uint32_t j = 0; j < PER; ++j) s += s_kept[scan_pad(threadIdx.x * PER + j)];
-        uint32_t total;
-        uint32_t run = carry + block_exclusive_scan(s, scratch, &total);
-#pragma unroll
-        for (uint32_t j = 0; j < PER; ++j) {
-            const uint32_t x = s_kept[scan_pad(threadIdx.x * PER + j)];
-            s_kept[scan_pad(threadIdx.x * PER + j)] = run;
-            run += x;
-        }
-        __syncthreads();
-        const uint32_t end = carry + total;  // offset just past this chunk
-#pragma unroll 4
-        for (uint32_t j = 0; j < PER; ++j) {
-            const uint32_t q = j * B + threadIdx.x;
-            if (q < cn) {
-                const uint32_t o = s_kept[scan_pad(q)];
-                const uint32_t o_next = q + 1 < cn ? s_kept[scan_pad(q + 1)] : end;
-                offset[c0 + q] = o;
-                recs[c0 + q] = make_uint4(o, o_next - o, 0u, 0u);
-            }
-        }
-        carry = end;
-        __syncthreads();  // s_kept is reused by the next chunk
+    __syncthreads();
+    block_scan_array(s_kept, int(m), s_scan);
+    for (uint32_t q = threadIdx.x; q < m; q += 256) {
+        const uint32_t o = s_kept[q];
+        p.offset[t0 + q] = o;
+        p.recs[t0 + q] = make_uint4(o, s_kept[q + 1] - o, 0u, 0u);
+        p.staged[t0 + q] = 0u;
     }
+    if (threadIdx.x == 0) {
+        p.run_total[blockIdx.x] = s_kept[m];
+        if (blockIdx.x == 0) p.ticket[0] = 0ull;
+        s_last = atom_add_acq_rel(reinterpret_cast<uint32_t*>(&p.ticket[1]), 1u) == gridDim.x - 1u ? 1u : 0u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    const uint32_t runs = gridDim.x;
+    for (uint32_t q = threadIdx.x; q < runs; q += 256) s_kept[q] = __ldcg(&p.run_total[q]);
+    __syncthreads();
+    block_scan_array(s_kept, int(runs), s_scan);
+    for (uint32_t q = threadIdx.x; q < runs; q += 256) p.run_recs[q] = make_uint4(s_kept[q], 0u, 0u, 0u);
+    if (threadIdx.x == 0) p.ticket[1] = 0ull;
 }
 
 // One tile per CTA, taken in ticket order (used for payloads that are not 16-byte aligned, and
 // when phase stamps are on).
 template <int W, int IPT>
 __global__ void __launch_bounds__(kPartBlock) partition_move_kernel(
-    uint8_t* data, uint32_t n, uint32_t ntiles, uint32_t* __restrict__ bits, const uint32_t* __restrict__ offset,
-    uint32_t* staged, unsigned long long* ticket, uint32_t tag, uint32_t* status, uint32_t spin_limit,
-    unsigned long long* dev_len, uint32_t new_len, unsigned long long* stamps, uint32_t stamp_stride) {
+    uint8_t* data, uint32_t n, uint32_t ntiles, uint32_t* __restrict__ bits, const PartScratch p, uint32_t run,
+    uint32_t tag, uint32_t* status, uint32_t spin_limit, unsigned long long* dev_len, uint32_t new_len, unsigned long long* stamps, uint32_t stamp_stride) {
     using T = typename Payload<W>::T;
+    uint32_t* staged = p.staged;
     T* A = reinterpret_cast<T*>(data);
     constexpr int B = kPartBlock, NW = B / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -152,7 +148,7 @@ __global__ void __launch_bounds__(kPartBlock) partition_move_kernel(
     if (blockIdx.x == 0 && threadIdx.x == 0 && dev_len) *dev_len = new_len;
     const unsigned long long t_start = stamps ? globaltimer() : 0ull;
 
-    if (threadIdx.x == 0) s_tile = uint32_t(atomicAdd(ticket, 1ull));
+    if (threadIdx.x == 0) s_tile = uint32_t(atomicAdd(p.ticket, 1ull));
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile >= ntiles) return;
@@ -164,7 +160,7 @@ __global__ void __launch_bounds__(kPartBlock) partition_move_kernel(
         my_stamps[1] = globaltimer();
     }
     const uint32_t base = tile * TILE;
-    const uint32_t off = __ldg(&offset[tile]);
+    const uint32_t off = __ldg(&p.run_recs[tile / run].x) + __ldg(&p.offset[tile]);
     T v[IPT];
     uint32_t wd[IPT];
 #pragma unroll
@@ -258,15 +254,16 @@ constexpr int kMoveBlock = kMoveGroups * kGroupThreads + 32;
 
 template <int W>
 constexpr size_t move_smem_bytes() {
-    return size_t(kMoveStages) * kTileBytes + size_t(kMoveStages) * (kTileBytes / W / 8) + size_t(kMoveStages) * 16;
+    return size_t(kMoveStages) * kTileBytes + size_t(kMoveStages) * (kTileBytes / W / 8) + size_t(kMoveStages) * 32;
 }
 
 template <int W>
 __global__ void __launch_bounds__(kMoveBlock, 1) partition_move_ws_kernel(
-    uint8_t* data, uint32_t n, uint32_t ntiles, uint32_t* __restrict__ bits, const uint4* __restrict__ recs,
-    uint32_t* staged, unsigned long long* ticket, uint32_t tag, uint32_t* status, uint32_t spin_limit,
-    unsigned long long* dev_len, uint32_t new_len) {
+    uint8_t* data, uint32_t n, uint32_t ntiles, uint32_t* __restrict__ bits, const PartScratch sc, uint32_t run,
+    uint32_t tag, uint32_t* status, uint32_t spin_limit, unsigned long long* dev_len, uint32_t new_len) {
     using T = typename Payload<W>::T;
+    uint32_t* staged = sc.staged;
+    unsigned long long* ticket = sc.ticket;
     constexpr uint32_t TILE = kTileBytes / W;  // items per tile
     constexpr uint32_t BW = TILE / 32;         // bitmap words per tile
     constexpr int S = kMoveStages;
@@ -280,7 +277,7 @@ __global__ void __launch_bounds__(kMoveBlock, 1) partition_move_ws_kernel(
     extern __shared__ __align__(128) uint8_t smem[];
     T* stage = reinterpret_cast<T*>(smem);                                   // [S][TILE]
     uint32_t* sbits = reinterpret_cast<uint32_t*>(smem + S * kTileBytes);    // [S][BW]
-    uint4* srec = reinterpret_cast<uint4*>(smem + S * kTileBytes + S * BW * 4);  // [S]
+    uint4* srec = reinterpret_cast<uint4*>(smem + S * kTileBytes + S * BW * 4);  // [S][2]: tile, run
     __shared__ __align__(8) unsigned long long full[S], empty[S];
     __shared__ uint32_t s_tile[S];
     __shared__ uint32_t s_wtot[kMoveGroups][GW];
@@ -330,10 +327,11 @@ __global__ void __launch_bounds__(kMoveBlock, 1) partition_move_ws_kernel(
                         const uint32_t base = t * TILE;
                         const uint32_t items = min(TILE, n - base);
                         const uint32_t bulk = (items * W) & ~15u;
-                        mbar_arrive_expect_tx(&full[s], bulk + BW * 4 + 16);
+                        mbar_arrive_expect_tx(&full[s], bulk + BW * 4 + 32);
                         if (bulk) tma_load_1d(stage + size_t(s) * TILE, data + size_t(base) * W, bulk, &full[s]);
                         tma_load_1d(sbits + s * BW, bits + size_t(t) * BW, BW * 4, &full[s]);
-                        tma_load_1d(&srec[s], recs + t, 16, &full[s]);
+                        tma_load_1d(&srec[2 * s], sc.recs + t, 16, &full[s]);
+                        tma_load_1d(&srec[2 * s + 1], sc.run_recs + t / run, 16, &full[s]);
                     } else {
                         done = true;
                         ++ends;
@@ -393,8 +391,8 @@ __global__ void __launch_bounds__(kMoveBlock, 1) partition_move_ws_kernel(
         if (t >= ntiles) break;
         const uint32_t base = t * TILE;
         const uint32_t items = min(TILE, n - base);
-        const uint4 rec = srec[s];
-        const uint32_t off = rec.x, total = rec.y;
+        const uint4 rec = srec[2 * s];
+        const uint32_t off = srec[2 * s + 1].x + rec.x, total = rec.y;
         T* st = stage + size_t(s) * TILE;
         // The ragged end of the last tile (fewer than 16 bytes) comes through plain loads.
         const uint32_t bulk_items = ((items * W) & ~15u) / W;
@@ -448,10 +446,10 @@ __global__ void __launch_bounds__(kMoveBlock, 1) partition_move_ws_kernel(
     }
 }
 
-using MoveFn = void (*)(uint8_t*, uint32_t, uint32_t, uint32_t*, const uint32_t*, uint32_t*, unsigned long long*,
-                        uint32_t, uint32_t*, uint32_t, unsigned long long*, uint32_t, unsigned long long*, uint32_t);
-using MoveWsFn = void (*)(uint8_t*, uint32_t, uint32_t, uint32_t*, const uint4*, uint32_t*, unsigned long long*,
-                          uint32_t, uint32_t*, uint32_t, unsigned long long*, uint32_t);
+using MoveFn = void (*)(uint8_t*, uint32_t, uint32_t, uint32_t*, PartScratch, uint32_t, uint32_t, uint32_t*, uint32_t,
+                        unsigned long long*, uint32_t, unsigned long long*, uint32_t);
+using MoveWsFn = void (*)(uint8_t*, uint32_t, uint32_t, uint32_t*, PartScratch, uint32_t, uint32_t, uint32_t*, uint32_t,
+                          unsigned long long*, uint32_t);
 
 // 32 KB of payload per tile for every width.
 static int part_items(int w) { return w == 4 ? 16 : w == 8 ? 8 : w == 16 ? 4 : 2; }
@@ -483,36 +481,34 @@ int launch_partition(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint
     st = reset_if_dirty(ctx, s);
     if (st != RZ_OK) return st;
     const bool validate = (flags & RZ_VALIDATE) != 0;
-    // Scratch layout in tile_state: the ticket on its own 128-byte line, then staged, kept and
-    // offset as 32-bit arrays of ntiles rounded up to a multiple of 4, then the 16-byte records.
-    // Ticket and staged flags are cleared by one memset per call (which keeps the call correct
-    // when it is replayed from a CUDA graph).
+    // Scratch layout in tile_state: the ticket on its own 128-byte line, then staged and offset as
+    // 32-bit arrays of ntiles rounded up to a multiple of 4, the tiles' and the runs' 16-byte records,
+    // and the runs' totals.
     const uint32_t ntp = (ntiles + 3u) & ~3u;
-    unsigned long long* ticket = ctx->ws.tile_state;
-    uint32_t* staged = reinterpret_cast<uint32_t*>(ctx->ws.tile_state + 16);
-    uint32_t* kept = staged + ntp;
-    uint32_t* offset = kept + ntp;
-    uint4* recs = reinterpret_cast<uint4*>(offset + ntp);
+    PartScratch sc;
+    sc.ticket = ctx->ws.tile_state;
+    sc.staged = reinterpret_cast<uint32_t*>(ctx->ws.tile_state + 16);
+    sc.offset = sc.staged + ntp;
+    sc.recs = reinterpret_cast<uint4*>(sc.offset + ntp);
+    sc.run_recs = sc.recs + ntiles;
+    sc.run_total = reinterpret_cast<uint32_t*>(sc.run_recs + kPartMaxRuns);
     const uint32_t tag = 1u;
-    RZ_CUDA_TRY(ctx, cudaMemsetAsync(ticket, 0, 128 + size_t(ntiles) * 4, s));
-    const int mgrid = std::max(1, std::min<int>(ctx->sms * 8, int((k + 255) / 256)));
-    partition_mark_kernel<<<mgrid, 256, 0, s>>>(idx, k, n, ctx->ws.part_bits, ctx->ws.status, validate ? 1u : 0u);
-    const int cgrid = std::max(1, std::min<int>(ctx->sms * 8, int((ntiles + 7) / 8)));
+    const int mgrid = int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(ctx->sms) * 8, (uint64_t(k) + 255) / 256)));
+    if (validate) partition_mark_kernel<true><<<mgrid, 256, 0, s>>>(idx, k, n, ctx->ws.part_bits, ctx->ws.status);
+    else partition_mark_kernel<false><<<mgrid, 256, 0, s>>>(idx, k, n, ctx->ws.part_bits, ctx->ws.status);
+    // Runs of 8 tiles (one per warp) or more, about four blocks per SM; kPartMaxRun * kPartMaxRuns tiles
+    // are more than any list has (n < 2^32 items of 32 bytes: 2^22 tiles).
+    const uint32_t most = std::max<uint32_t>(uint32_t(ctx->sms) * 4, (ntiles + kPartMaxRun - 1) / kPartMaxRun);
+    const uint32_t run = std::max<uint32_t>((ntiles + most - 1) / most, std::min<uint32_t>(8, ntiles));
+    const uint32_t cgrid = (ntiles + run - 1) / run;
+    uint32_t* bits = ctx->ws.part_bits;
     switch (w) {
-        case 4: partition_count_kernel<kTileBytes / 4 / 32><<<cgrid, 256, 0, s>>>(ctx->ws.part_bits, n, ntiles, kept); break;
-        case 8: partition_count_kernel<kTileBytes / 8 / 32><<<cgrid, 256, 0, s>>>(ctx->ws.part_bits, n, ntiles, kept); break;
-        case 16: partition_count_kernel<kTileBytes / 16 / 32><<<cgrid, 256, 0, s>>>(ctx->ws.part_bits, n, ntiles, kept); break;
-        default: partition_count_kernel<kTileBytes / 32 / 32><<<cgrid, 256, 0, s>>>(ctx->ws.part_bits, n, ntiles, kept); break;
+        case 4: partition_count_kernel<kTileBytes / 4 / 32><<<cgrid, 256, 0, s>>>(bits, n, ntiles, run, sc); break;
+        case 8: partition_count_kernel<kTileBytes / 8 / 32><<<cgrid, 256, 0, s>>>(bits, n, ntiles, run, sc); break;
+        case 16: partition_count_kernel<kTileBytes / 16 / 32><<<cgrid, 256, 0, s>>>(bits, n, ntiles, run, sc); break;
+        default: partition_count_kernel<kTileBytes / 32 / 32><<<cgrid, 256, 0, s>>>(bits, n, ntiles, run, sc); break;
     }
-    // Function attributes belong to a device: one bit per device (first 64 devices).
-    static std::atomic<uint64_t> scan_attr{0};
-    const uint64_t dev_bit = 1ull << (ctx->device & 63);
-    if (!(scan_attr.load() & dev_bit)) {
-        RZ_CUDA_TRY(ctx, cudaFuncSetAttribute((const void*)partition_scan_kernel,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, int(kScanSmem)));
-        scan_attr.fetch_or(dev_bit);
-    }
-    partition_scan_kernel<<<1, 1024, kScanSmem, s>>>(kept, ntiles, offset, recs);
+    const uint64_t dev_bit = 1ull << (ctx->device & 63);  // function attributes belong to a device (first 64)
     int grid = int(ntiles), block = kPartBlock;
     if ((reinterpret_cast<uintptr_t>(data) & 15u) == 0 && !ctx->ws.stamps_on) {
         size_t smem = 0;
@@ -525,13 +521,12 @@ int launch_partition(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint
         }
         grid = std::max(1, std::min<int>(ctx->sms, int(ntiles)));
         block = kMoveBlock;
-        f<<<grid, kMoveBlock, smem, s>>>(static_cast<uint8_t*>(data), n, ntiles, ctx->ws.part_bits, recs, staged,
-                                         ticket, tag, ctx->ws.status, kSpinLimit, ctx->ws.dev_len, n - k);
+        f<<<grid, kMoveBlock, smem, s>>>(static_cast<uint8_t*>(data), n, ntiles, bits, sc, run, tag, ctx->ws.status,
+                                         kSpinLimit, ctx->ws.dev_len, n - k);
     } else {
         const uint32_t stride = std::max<uint32_t>(1u, (ntiles + kMaxGrid - 1) / kMaxGrid);
         move_fn(int(w))<<<ntiles, kPartBlock, 0, s>>>(
-            static_cast<uint8_t*>(data), n, ntiles, ctx->ws.part_bits, offset, staged, ticket, tag, ctx->ws.status,
-            kSpinLimit, ctx->ws.dev_len, n - k, ctx->ws.stamps_on ? ctx->ws.stamps : nullptr, stride);
+            static_cast<uint8_t*>(data), n, ntiles, bits, sc, run, tag, ctx->ws.status, kSpinLimit, ctx->ws.dev_len, n - k, ctx->ws.stamps_on ? ctx->ws.stamps : nullptr, stride);
         grid = std::min<int>(int(ntiles), kMaxGrid);
     }
     RZ_CUDA_TRY(ctx, cudaGetLastError());
@@ -539,7 +534,7 @@ int launch_partition(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint
         info->grid = grid;
         info->block = block;
         info->items = items;
-        info->launches += 4;  // mark, count, scan, move (the ticket memset runs on the copy engine)
+        info->launches += 3;  // mark, count, move
     }
     return RZ_OK;
 }

@@ -108,3 +108,27 @@ def test_validation_both_ways(ctx, n, share):
         exp = host.copy()
         oracle.remove(exp, good)
         assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n - k], exp[: n - k])
+
+
+@pytest.mark.parametrize("words", [1, 8])
+@pytest.mark.parametrize("n_tiles,extra", [(1, -3), (1, 0), (8, 0), (8, 1), (9, 0), (600, 17), (1191, 5)])
+def test_partition_runs_of_tiles(ctx, words, n_tiles, extra):
+    """The partition's tiles are counted in runs: sizes around one tile, one run (8 tiles, or 3 at
+    about 1200) and a last run that is cut short; an aligned list (pipelined move) and, for 4-byte
+    items, one that is not; validated and not; twice on the same context."""
+    n = n_tiles * (32768 // (4 * words)) + extra
+    k = n // 7
+    rng = np.random.default_rng(n + words)
+    host = payload(n, words, seed=n)
+    idx = rng.choice(n, size=k, replace=False).astype(np.uint32)
+    exp = np.delete(host, idx.astype(np.int64), axis=0)
+    d_idx = on_gpu(idx)
+    for flags in (rz.RZ_SYNC, rz.RZ_SYNC | rz.RZ_VALIDATE):
+        d = on_gpu(host)
+        assert ctx.partition(d, d_idx, flags=flags) == n - k
+        assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n - k], exp)
+    if words == 1:
+        room = torch.zeros((n + 1, 1), dtype=torch.int32, device=DEV)
+        room[1:] = on_gpu(host)
+        assert ctx.partition(room[1:], d_idx, flags=rz.RZ_SYNC) == n - k
+        assert np.array_equal(room[1: n - k + 1].cpu().numpy().view(np.uint32), exp)
