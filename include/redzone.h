@@ -172,7 +172,8 @@ int rz_keep(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, const uin
  *   rz_keyindex_build  -- clear, then index rows [0, n); RZ_ERR_DUPLICATE on a repeated key.
  *   rz_keyindex_insert -- index rows [first, first + count) (e.g. after rz_append_remove); the
  *                         keys must not be indexed already. Both are synchronous.
- *   rz_keyindex_find   -- rows of `count` keys into d_rows (0xffffffff when absent), async.
+ *   rz_keyindex_find   -- rows of `count` keys into d_rows (0xffffffff when absent), async;
+ *   rz_keyindex_find64 -- the same as 64-bit rows, -1 when absent.
  *   rz_remove_by_key   -- remove the rows holding the k given keys with the Redzone rule and keep
  *                         the index exact: deleted keys are erased and each item moved into a hole
  *                         is re-pointed at it (O(k); no other row changes). Synchronous up to the
@@ -186,6 +187,7 @@ int rz_keyindex_build(rz_keyindex* ix, const void* d_data, int64_t n, uint32_t r
 int rz_keyindex_insert(rz_keyindex* ix, const void* d_data, int64_t first, int64_t count, uint32_t record_bytes,
                        rz_stream_t stream);
 int rz_keyindex_find(rz_keyindex* ix, const uint64_t* d_keys, int64_t count, uint32_t* d_rows, rz_stream_t stream);
+int rz_keyindex_find64(rz_keyindex* ix, const uint64_t* d_keys, int64_t count, int64_t* d_rows, rz_stream_t stream);
 int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint32_t record_bytes,
                      const uint64_t* d_keys, int64_t k, int64_t* new_len, uint32_t flags, rz_stream_t stream);
 

@@ -314,13 +314,10 @@ class KeyIndex:
     def find(self, keys, stream=None):
         """Rows (int64 tensor, -1 when absent) of a CUDA int64 tensor of keys."""
         import torch
-        rows = torch.empty(keys.numel(), dtype=torch.int32, device=keys.device)
-        self.ctx._check(_native.lib.rz_keyindex_find(self.handle, ctypes.c_void_p(keys.data_ptr()), keys.numel(),
-                                                     ctypes.c_void_p(rows.data_ptr()),
-                                                     ctypes.c_void_p(_stream_handle(stream))), "rz_keyindex_find")
-        r = rows.to(torch.int64) & 0xFFFFFFFF
-        r[r == 0xFFFFFFFF] = -1
-        return r
+        rows = torch.empty(keys.numel(), dtype=torch.int64, device=keys.device)
+        self.ctx._check(_native.lib.rz_keyindex_find64(self.handle, keys.data_ptr(), keys.numel(), rows.data_ptr(),
+                                                       _stream_handle(stream)), "rz_keyindex_find64")
+        return rows
 
     def remove_by_key(self, table, n: int, keys, flags: int = 0, stream=None) -> int:
         out = ctypes.c_int64(0)

@@ -105,6 +105,7 @@ _sig("rz_keyindex_destroy", None, [c_vp])
 _sig("rz_keyindex_build", c_i32, [c_vp, c_vp, c_i64, c_u32, c_vp])
 _sig("rz_keyindex_insert", c_i32, [c_vp, c_vp, c_i64, c_i64, c_u32, c_vp])
 _sig("rz_keyindex_find", c_i32, [c_vp, c_vp, c_i64, c_vp, c_vp])
+_sig("rz_keyindex_find64", c_i32, [c_vp, c_vp, c_i64, c_vp, c_vp])
 _sig("rz_remove_by_key", c_i32, [c_vp, c_vp, c_vp, c_i64, c_u32, c_vp, c_i64, ctypes.POINTER(c_i64), c_u32, c_vp])
 _sig("rz_partition", c_i32, [c_vp, c_vp, c_i64, c_u32, c_vp, c_i64, ctypes.POINTER(c_i64), c_u32, c_vp])
 _sig("rz_default_cfg", c_i32, [c_vp, c_i64, c_i64, c_u32, ctypes.POINTER(LaunchCfg)])

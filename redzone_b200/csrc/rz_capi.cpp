@@ -127,12 +127,27 @@ int wait_event(rz_ctx* ctx, cudaEvent_t ev) {
     return RZ_OK;
 }
 
-static int fetch_result(rz_ctx* ctx, cudaStream_t s, uint32_t* status, unsigned long long* len) {
+int queue_status(rz_ctx* ctx, cudaStream_t s) {
     RZ_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->ws.h_result, ctx->ws.status, kResultBytes, cudaMemcpyDeviceToHost, s));
     RZ_CUDA_TRY(ctx, cudaEventRecord(ctx->done_event, s));
+    return RZ_OK;
+}
+
+int await_status(rz_ctx* ctx, uint32_t* status) {
     const int st = wait_event(ctx, ctx->done_event);
     if (st != RZ_OK) return st;
     std::memcpy(status, ctx->ws.h_result, sizeof(uint32_t));
+    return RZ_OK;
+}
+
+int fetch_status(rz_ctx* ctx, cudaStream_t s, uint32_t* status) {
+    const int st = queue_status(ctx, s);
+    return st != RZ_OK ? st : await_status(ctx, status);
+}
+
+static int fetch_result(rz_ctx* ctx, cudaStream_t s, uint32_t* status, unsigned long long* len) {
+    const int st = fetch_status(ctx, s, status);
+    if (st != RZ_OK) return st;
     if (len) std::memcpy(len, ctx->ws.h_result + 512, sizeof(unsigned long long));
     return RZ_OK;
 }
@@ -160,6 +175,61 @@ static int check_args(const void* data, int64_t n, uint32_t w, const uint32_t* i
     if (reinterpret_cast<uintptr_t>(data) % align) return RZ_ERR_INVALID_ARG;
     if (reinterpret_cast<uintptr_t>(idx) % 4) return RZ_ERR_INVALID_ARG;
     return RZ_OK;
+}
+
+static int remove_cfg(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, const uint32_t* d_idx, int64_t k,
+                      const rz_launch_cfg* cfg, uint32_t flags, rz_stream_t stream) {
+    if (!ctx || !cfg) return RZ_ERR_INVALID_ARG;
+    int st = check_args(d_data, n, elem_bytes, d_idx, k);
+    if (st != RZ_OK) return st;
+    std::lock_guard<std::recursive_mutex> g(ctx->mu);
+    cudaSetDevice(ctx->device);
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    ctx->last_kernels = 0;
+    ctx->last_grid = 0;
+    ctx->last_block = 0;
+    if (k == 0 || k == n) {
+        // Nothing moves (reference: redzone.hxx:651, Redzone_CPU.hxx handles it implicitly).
+        if ((flags & RZ_VALIDATE) && !(flags & kPrevalidated) && k > 0) {
+            st = launch_validate(ctx, uint32_t(n), d_idx, uint32_t(k), s);
+            if (st != RZ_OK) return st;
+            ctx->last_kernels = 2;
+        }
+        return (flags & RZ_SYNC) ? read_status(ctx, s) : RZ_OK;
+    }
+    LaunchInfo info;
+    if (cfg->use_partition || (flags & RZ_FORCE_PARTITION))
+        st = launch_partition(ctx, d_data, uint32_t(n), elem_bytes, d_idx, uint32_t(k), flags, s, &info);
+    else
+        st = launch_redzone(ctx, d_data, uint32_t(n), elem_bytes, d_idx, uint32_t(k), *cfg, flags, s, &info);
+    if (st != RZ_OK) return st;
+    ctx->last_kernels = info.launches;
+    ctx->last_grid = info.grid;
+    ctx->last_block = info.block;
+    return (flags & RZ_SYNC) ? read_status(ctx, s) : RZ_OK;
+}
+
+int remove_impl(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, const uint32_t* d_idx, int64_t k,
+                int64_t* new_len, uint32_t flags, rz_stream_t stream) {
+    if (!ctx) return RZ_ERR_INVALID_ARG;
+    int st = check_args(d_data, n, elem_bytes, d_idx, k);
+    if (st != RZ_OK) return st;
+    if (new_len) *new_len = n - k;
+    std::lock_guard<std::recursive_mutex> g(ctx->mu);
+    cudaSetDevice(ctx->device);
+    rz_launch_cfg cfg{};
+    bool have = false;
+    if (flags & RZ_USE_PREDICTOR)
+        have = predict_cfg(ctx, uint32_t(n), uint32_t(k), elem_bytes, d_idx,
+                              reinterpret_cast<cudaStream_t>(stream), &cfg);
+    if (!have) have = tuned_cfg(ctx, uint32_t(n), uint32_t(k), elem_bytes, &cfg);
+    if (!have) {
+        st = default_cfg(ctx, uint32_t(n), uint32_t(k), elem_bytes, &cfg);
+        if (st != RZ_OK) return st;
+    }
+    // The partition path reorders survivors; it runs only when the caller allows that order.
+    if (cfg.use_partition && !(flags & RZ_ALLOW_STABLE)) cfg.use_partition = 0;
+    return remove_cfg(ctx, d_data, n, elem_bytes, d_idx, k, &cfg, flags, stream);
 }
 
 }  // namespace rz
@@ -308,57 +378,12 @@ int rz_default_cfg(const rz_ctx* ctx, int64_t n, int64_t k, uint32_t elem_bytes,
 
 int rz_remove_cfg(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, const uint32_t* d_idx,
                   int64_t k, const rz_launch_cfg* cfg, uint32_t flags, rz_stream_t stream) {
-    if (!ctx || !cfg) return RZ_ERR_INVALID_ARG;
-    int st = check_args(d_data, n, elem_bytes, d_idx, k);
-    if (st != RZ_OK) return st;
-    std::lock_guard<std::recursive_mutex> g(ctx->mu);
-    cudaSetDevice(ctx->device);
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    ctx->last_kernels = 0;
-    ctx->last_grid = 0;
-    ctx->last_block = 0;
-    if (k == 0 || k == n) {
-        // Nothing moves (reference: redzone.hxx:651, Redzone_CPU.hxx handles it implicitly).
-        if (flags & RZ_VALIDATE && k > 0) {
-            st = launch_validate(ctx, uint32_t(n), d_idx, uint32_t(k), s);
-            if (st != RZ_OK) return st;
-            ctx->last_kernels = 2;
-        }
-        return (flags & RZ_SYNC) ? read_status(ctx, s) : RZ_OK;
-    }
-    LaunchInfo info;
-    if (cfg->use_partition || (flags & RZ_FORCE_PARTITION))
-        st = launch_partition(ctx, d_data, uint32_t(n), elem_bytes, d_idx, uint32_t(k), flags, s, &info);
-    else
-        st = launch_redzone(ctx, d_data, uint32_t(n), elem_bytes, d_idx, uint32_t(k), *cfg, flags, s, &info);
-    if (st != RZ_OK) return st;
-    ctx->last_kernels = info.launches;
-    ctx->last_grid = info.grid;
-    ctx->last_block = info.block;
-    return (flags & RZ_SYNC) ? read_status(ctx, s) : RZ_OK;
+    return remove_cfg(ctx, d_data, n, elem_bytes, d_idx, k, cfg, flags & ~kPrevalidated, stream);
 }
 
 int rz_remove(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, const uint32_t* d_idx, int64_t k,
               int64_t* new_len, uint32_t flags, rz_stream_t stream) {
-    if (!ctx) return RZ_ERR_INVALID_ARG;
-    int st = check_args(d_data, n, elem_bytes, d_idx, k);
-    if (st != RZ_OK) return st;
-    if (new_len) *new_len = n - k;
-    std::lock_guard<std::recursive_mutex> g(ctx->mu);
-    cudaSetDevice(ctx->device);
-    rz_launch_cfg cfg{};
-    bool have = false;
-    if (flags & RZ_USE_PREDICTOR)
-        have = predict_cfg(ctx, uint32_t(n), uint32_t(k), elem_bytes, d_idx,
-                              reinterpret_cast<cudaStream_t>(stream), &cfg);
-    if (!have) have = tuned_cfg(ctx, uint32_t(n), uint32_t(k), elem_bytes, &cfg);
-    if (!have) {
-        st = default_cfg(ctx, uint32_t(n), uint32_t(k), elem_bytes, &cfg);
-        if (st != RZ_OK) return st;
-    }
-    // The partition path reorders survivors; it runs only when the caller allows that order.
-    if (cfg.use_partition && !(flags & RZ_ALLOW_STABLE)) cfg.use_partition = 0;
-    return rz_remove_cfg(ctx, d_data, n, elem_bytes, d_idx, k, &cfg, flags, stream);
+    return remove_impl(ctx, d_data, n, elem_bytes, d_idx, k, new_len, flags & ~kPrevalidated, stream);
 }
 
 int rz_append_remove(rz_ctx* ctx, void* d_data, int64_t n, int64_t capacity, uint32_t elem_bytes,

@@ -164,6 +164,16 @@ void release_extras(rz_ctx* ctx);
 constexpr size_t kResultBytes = 512 + sizeof(unsigned long long);
 // Wait for an event: poll (about 2 ms), then block. RZ_OK or RZ_ERR_CUDA.
 int wait_event(rz_ctx* ctx, cudaEvent_t ev);
+// The status word and the device length, copied behind what is queued on the stream (the event is
+// recorded after the copy); wait for that copy; both.
+int queue_status(rz_ctx* ctx, cudaStream_t s);
+int await_status(rz_ctx* ctx, uint32_t* status);
+int fetch_status(rz_ctx* ctx, cudaStream_t s, uint32_t* status);
+// With RZ_VALIDATE: the list was checked by the library itself, and the status word says how that went.
+constexpr uint32_t kPrevalidated = 1u << 31;
+// rz_remove, which also takes kPrevalidated.
+int remove_impl(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, const uint32_t* d_idx, int64_t k,
+                int64_t* new_len, uint32_t flags, rz_stream_t stream);
 // Map device status bits (ST_* of rz_common.cuh) to an rz_status code, most severe first.
 int map_status(uint32_t bits);
 // Wait for the stream, then map the device status to rz_status (clearing it); with new_len, also

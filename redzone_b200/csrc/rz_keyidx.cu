@@ -8,6 +8,14 @@
 // Removal by key keeps the index exact in O(k): the canonical rule moves an item only into a hole
 // below the cut (every other surviving item keeps its row), so after the removal each hole's new
 // occupant is re-pointed at the hole, and the deleted keys are erased. Nothing is rescanned.
+// The lookup also claims each slot it finds (one bit), which catches a key given twice; a missing or repeated
+// key goes into the context's status word, which the removal (as after RZ_VALIDATE's passes) and the
+// index update look at before they change anything. So the whole call is queued at once and the host
+// waits for it once. Bound by the random accesses of the probes and by that wait: deleting 65521 of
+// 4.2M 32-byte records by key, inserting as many and looking as many up takes 97 us, and took 165 us
+// with a wait after the lookup, validation passes over the rows, and 64-bit rows made from 32-bit ones
+// by the caller. (Keys and rows in one 16-byte slot made the calls 7 % faster but the build slower by
+// half: 134 MB of slots do not stay in L2.)
 #include <algorithm>
 #include <new>
 
@@ -19,7 +27,7 @@ namespace rz {
 constexpr unsigned long long kEmptyKey = ~0ull;
 constexpr unsigned long long kErasedKey = ~0ull - 1ull;
 constexpr uint32_t kNoRow = 0xffffffffu;
-enum : uint32_t { IX_DUPLICATE = 1u, IX_MISSING = 2u, IX_FULL = 4u, IX_RESERVED = 8u };
+enum : uint32_t { IX_DUPLICATE = 1u, IX_FULL = 4u, IX_RESERVED = 8u };  // status bits of an insert
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
@@ -73,37 +81,59 @@ __global__ void ix_insert_kernel(unsigned long long* keys, uint32_t* rows, uint3
     }
 }
 
-// Rows of the keys to delete (kNoRow and IX_MISSING when absent) and their slots.
-__global__ void ix_lookup_kernel(const unsigned long long* keys, const uint32_t* rows, uint32_t mask,
-                                 const unsigned long long* q, uint32_t count, uint32_t* out_rows,
-                                 uint32_t* out_slots, uint32_t* status) {
+// Rows of the keys asked for; when absent kNoRow, or -1 in 64 bits.
+template <typename Row>
+__global__ void ix_find_kernel(const unsigned long long* keys, const uint32_t* rows, uint32_t mask,
+                               const unsigned long long* q, uint32_t count, Row* out_rows) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const unsigned long long key = q[i];
         const uint32_t s = key >= kErasedKey ? kNoRow : find_slot(keys, mask, key);
-        if (s == kNoRow) {
-            out_rows[i] = kNoRow;
-            if (out_slots) atomicOr(status, IX_MISSING);
-        } else {
-            out_rows[i] = rows[s];
-        }
-        if (out_slots) out_slots[i] = s;
+        out_rows[i] = s == kNoRow ? Row(-1) : Row(rows[s]);
     }
 }
 
-__global__ void ix_erase_kernel(unsigned long long* keys, const uint32_t* slots, uint32_t count) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-        keys[slots[i]] = kErasedKey;
+// Rows and slots of the keys to delete (kNoRow when absent); every slot is claimed. A missing key
+// is an entry outside the list (ST_RANGE), one given twice a duplicate.
+__global__ void ix_claim_kernel(const unsigned long long* keys, const uint32_t* rows, uint32_t* claims, uint32_t mask,
+                                const unsigned long long* q, uint32_t count, uint32_t* out_rows, uint32_t* out_slots,
+                                uint32_t* status) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const unsigned long long key = q[i];
+        const uint32_t s = key >= kErasedKey ? kNoRow : find_slot(keys, mask, key);
+        uint32_t row = kNoRow;
+        if (s == kNoRow) {
+            atomicOr(status, ST_RANGE);
+        } else {
+            row = rows[s];
+            const uint32_t bit = 1u << (s & 31u);
+            if (atomicOr(&claims[s >> 5], bit) & bit) atomicOr(status, ST_DUPLICATE);
+        }
+        out_rows[i] = row;
+        out_slots[i] = s;
+    }
 }
 
-// After the removal: every hole below the cut holds a moved item; point its key at the hole.
-__global__ void ix_repoint_kernel(const unsigned long long* keys, uint32_t* rows, uint32_t mask, const uint8_t* data,
-                                  uint32_t w, const uint32_t* holes, uint32_t count, uint32_t cut) {
+// After the removal, if it took place: erase the deleted keys, and point the key of the item that
+// moved into each hole below the cut at the hole (a live key, so its probe never ends at a slot
+// that is erased meanwhile).
+__global__ void ix_update_kernel(unsigned long long* keys, uint32_t* rows, uint32_t* claims, uint32_t mask,
+                                 const uint8_t* data, uint32_t w, const uint32_t* holes, const uint32_t* del_slots,
+                                 uint32_t count, uint32_t cut, const uint32_t* status) {
+    if (__ldcg(status) != 0u) return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const uint32_t h = holes[i];
+        const uint32_t h = holes[i], d = del_slots[i];
+        keys[d] = kErasedKey;
+        claims[d >> 5] = 0u;  // every claim in the word is this call's
         if (h >= cut) continue;
         const uint32_t s = find_slot(keys, mask, record_key(data, w, h));
         if (s != kNoRow) rows[s] = h;
     }
+}
+
+// A removal that did not take place lets go of its slots.
+__global__ void ix_unclaim_kernel(uint32_t* claims, const uint32_t* del_slots, uint32_t count) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+        if (del_slots[i] != kNoRow) claims[del_slots[i] >> 5] = 0u;
 }
 
 static int grid_for(const rz_ctx* ctx, int64_t count) {
@@ -116,11 +146,13 @@ struct rz_keyindex {
     rz_ctx* ctx = nullptr;
     unsigned long long* keys = nullptr;
     uint32_t* rows = nullptr;
+    uint32_t* claims = nullptr;      // one bit per slot, zero between calls
     uint32_t mask = 0;
     uint32_t* status = nullptr;      // device
     uint32_t* h_status = nullptr;    // pinned
     uint32_t* del_rows = nullptr;    // removal list of the current call
     uint32_t* del_slots = nullptr;
+    uint32_t* del_own = nullptr;     // their own allocation, once a removal outgrew the index's
     size_t del_cap = 0;
 };
 
@@ -128,7 +160,9 @@ using namespace rz;
 
 static int ix_status(rz_keyindex* ix, cudaStream_t s, uint32_t* bits) {
     RZ_CUDA_TRY(ix->ctx, cudaMemcpyAsync(ix->h_status, ix->status, 4, cudaMemcpyDeviceToHost, s));
-    RZ_CUDA_TRY(ix->ctx, cudaStreamSynchronize(s));
+    RZ_CUDA_TRY(ix->ctx, cudaEventRecord(ix->ctx->done_event, s));
+    const int st = wait_event(ix->ctx, ix->ctx->done_event);
+    if (st != RZ_OK) return st;
     *bits = *ix->h_status;
     if (*bits) RZ_CUDA_TRY(ix->ctx, cudaMemsetAsync(ix->status, 0, 4, s));
     return RZ_OK;
@@ -138,7 +172,20 @@ static int ix_map(uint32_t bits) {
     if (bits & IX_RESERVED) return RZ_ERR_INVALID_ARG;
     if (bits & IX_FULL) return RZ_ERR_NO_MEMORY;
     if (bits & IX_DUPLICATE) return RZ_ERR_DUPLICATE;
-    if (bits & IX_MISSING) return RZ_ERR_OUT_OF_RANGE;
+    return RZ_OK;
+}
+
+template <typename Row>
+static int ix_find(rz_keyindex* ix, const uint64_t* d_keys, int64_t count, Row* d_rows, rz_stream_t stream) {
+    if (!ix || count < 0 || (count > 0 && (!d_keys || !d_rows)) || count > (int64_t(1) << 32) - 1)
+        return RZ_ERR_INVALID_ARG;
+    rz_ctx* ctx = ix->ctx;
+    std::lock_guard<std::recursive_mutex> lock(ctx->mu);
+    cudaSetDevice(ctx->device);
+    if (count == 0) return RZ_OK;
+    ix_find_kernel<<<grid_for(ctx, count), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        ix->keys, ix->rows, ix->mask, reinterpret_cast<const unsigned long long*>(d_keys), uint32_t(count), d_rows);
+    RZ_CUDA_TRY(ctx, cudaGetLastError());
     return RZ_OK;
 }
 
@@ -156,17 +203,28 @@ int rz_keyindex_create(rz_ctx* ctx, int64_t capacity, rz_keyindex** out) {
     if (!ix) return RZ_ERR_NO_MEMORY;
     ix->ctx = ctx;
     ix->mask = uint32_t(cap - 1);
-    cudaError_t e = cudaMalloc(&ix->keys, cap * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&ix->rows, cap * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&ix->status, 4);
-    if (e == cudaSuccess) e = cudaMemset(ix->status, 0, 4);
+    // One allocation: keys | rows | claims | status | rows and slots of a removal of up to cap / 32 keys
+    // (a longer one gets arrays of its own; 2 % of the index).
+    // The removal list starts on 16 bytes, as the scanning schedules want it.
+    const size_t claim_words = ((cap + 31) / 32 + 3) & ~size_t(3), del = std::max<size_t>(size_t(cap / 32), 1024);
+    const size_t off_claims = (size_t(cap) * 12 + 15) & ~size_t(15);
+    uint8_t* mem = nullptr;
+    cudaError_t e = cudaMalloc(&mem, off_claims + (claim_words + 4 + 2 * del) * 4);
+    if (e == cudaSuccess) {
+        ix->keys = reinterpret_cast<unsigned long long*>(mem);
+        ix->rows = reinterpret_cast<uint32_t*>(ix->keys + cap);
+        ix->claims = reinterpret_cast<uint32_t*>(mem + off_claims);
+        ix->status = ix->claims + claim_words;
+        ix->del_rows = ix->status + 4;
+        ix->del_slots = ix->del_rows + del;
+        ix->del_cap = del;
+        e = cudaMemset(ix->claims, 0, (claim_words + 4) * 4);
+    }
     if (e == cudaSuccess) e = cudaMemset(ix->keys, 0xff, cap * 8);
     if (e == cudaSuccess) e = cudaMallocHost(&ix->h_status, 4);
     if (e != cudaSuccess) {
         const int st = cuda_fail(ctx, e, "rz_keyindex_create");
         cudaFree(ix->keys);
-        cudaFree(ix->rows);
-        cudaFree(ix->status);
         delete ix;
         return st;
     }
@@ -178,10 +236,7 @@ void rz_keyindex_destroy(rz_keyindex* ix) {
     if (!ix) return;
     cudaSetDevice(ix->ctx->device);
     cudaFree(ix->keys);
-    cudaFree(ix->rows);
-    cudaFree(ix->status);
-    cudaFree(ix->del_rows);
-    cudaFree(ix->del_slots);
+    cudaFree(ix->del_own);
     if (ix->h_status) cudaFreeHost(ix->h_status);
     delete ix;
 }
@@ -219,17 +274,11 @@ int rz_keyindex_build(rz_keyindex* ix, const void* d_data, int64_t n, uint32_t r
 }
 
 int rz_keyindex_find(rz_keyindex* ix, const uint64_t* d_keys, int64_t count, uint32_t* d_rows, rz_stream_t stream) {
-    if (!ix || count < 0 || (count > 0 && (!d_keys || !d_rows)) || count > (int64_t(1) << 32) - 1)
-        return RZ_ERR_INVALID_ARG;
-    rz_ctx* ctx = ix->ctx;
-    std::lock_guard<std::recursive_mutex> lock(ctx->mu);
-    cudaSetDevice(ctx->device);
-    if (count == 0) return RZ_OK;
-    ix_lookup_kernel<<<grid_for(ctx, count), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        ix->keys, ix->rows, ix->mask, reinterpret_cast<const unsigned long long*>(d_keys), uint32_t(count), d_rows,
-        nullptr, ix->status);
-    RZ_CUDA_TRY(ctx, cudaGetLastError());
-    return RZ_OK;
+    return ix_find(ix, d_keys, count, d_rows, stream);
+}
+
+int rz_keyindex_find64(rz_keyindex* ix, const uint64_t* d_keys, int64_t count, int64_t* d_rows, rz_stream_t stream) {
+    return ix_find(ix, d_keys, count, d_rows, stream);
 }
 
 int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint32_t record_bytes,
@@ -243,35 +292,49 @@ int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint
     if (new_len) *new_len = n - k;
     if (k == 0) return RZ_OK;
     if (size_t(k) > ix->del_cap) {
-        cudaFree(ix->del_rows);
-        cudaFree(ix->del_slots);
-        ix->del_rows = ix->del_slots = nullptr;
+        cudaFree(ix->del_own);
+        ix->del_own = ix->del_rows = ix->del_slots = nullptr;
         ix->del_cap = 0;
-        const size_t cap = std::max<size_t>(size_t(k), 1024);
-        RZ_CUDA_TRY(ctx, cudaMalloc(&ix->del_rows, cap * 4));
-        RZ_CUDA_TRY(ctx, cudaMalloc(&ix->del_slots, cap * 4));
+        const size_t cap = (size_t(k) + 3) & ~size_t(3);
+        RZ_CUDA_TRY(ctx, cudaMalloc(&ix->del_own, cap * 8));
+        ix->del_rows = ix->del_own;
+        ix->del_slots = ix->del_own + cap;
         ix->del_cap = cap;
     }
-    // 1. rows of the keys; any missing key fails the call before anything changes.
-    ix_lookup_kernel<<<grid_for(ctx, k), 256, 0, s>>>(ix->keys, ix->rows, ix->mask,
-                                                     reinterpret_cast<const unsigned long long*>(d_keys),
-                                                     uint32_t(k), ix->del_rows, ix->del_slots, ix->status);
+    int st = reset_if_dirty(ctx, s);
+    if (st != RZ_OK) return st;
+    const int grid = grid_for(ctx, k);
+    ix_claim_kernel<<<grid, 256, 0, s>>>(ix->keys, ix->rows, ix->claims, ix->mask,
+                                         reinterpret_cast<const unsigned long long*>(d_keys), uint32_t(k), ix->del_rows,
+                                         ix->del_slots, ctx->ws.status);
     RZ_CUDA_TRY(ctx, cudaGetLastError());
+    // The removal, unless the claims failed. A removal that may take the O(n) path knows no such
+    // refusal, and the predictor reads the rows: there the host looks at the outcome first.
+    const bool look = (flags & (RZ_FORCE_PARTITION | RZ_ALLOW_STABLE | RZ_USE_PREDICTOR)) != 0;
     uint32_t bits = 0;
-    int st = ix_status(ix, s, &bits);
-    if (st != RZ_OK) return st;
-    if (bits) return ix_map(bits);
-    // 2. the removal itself (duplicates among the keys give duplicate rows: RZ_VALIDATE catches
-    //    them before any data moves), then 3. erase the deleted keys and re-point the moved ones.
+    if (look) st = fetch_status(ctx, s, &bits);
     int64_t nl = 0;
-    st = rz_remove(ctx, d_data, n, record_bytes, ix->del_rows, k, &nl, (flags | RZ_VALIDATE) & ~RZ_SYNC, stream);
-    if (st != RZ_OK) return st;
-    st = read_status(ctx, s);
-    if (st != RZ_OK) return st;
-    ix_erase_kernel<<<grid_for(ctx, k), 256, 0, s>>>(ix->keys, ix->del_slots, uint32_t(k));
-    ix_repoint_kernel<<<grid_for(ctx, k), 256, 0, s>>>(ix->keys, ix->rows, ix->mask, static_cast<const uint8_t*>(d_data),
-                                                      record_bytes, ix->del_rows, uint32_t(k), uint32_t(n - k));
-    RZ_CUDA_TRY(ctx, cudaGetLastError());
+    if (st == RZ_OK && bits == 0)
+        st = remove_impl(ctx, d_data, n, record_bytes, ix->del_rows, k, &nl,
+                       ((flags & ~kPrevalidated) | RZ_VALIDATE | (look ? 0u : kPrevalidated)) & ~uint32_t(RZ_SYNC), stream);
+    // The status as the removal left it; the index update, which looks at it too, runs meanwhile.
+    if (st == RZ_OK && bits == 0) st = queue_status(ctx, s);
+    if (st == RZ_OK && bits == 0) {
+        ix_update_kernel<<<grid, 256, 0, s>>>(ix->keys, ix->rows, ix->claims, ix->mask,
+                                              static_cast<const uint8_t*>(d_data), record_bytes, ix->del_rows,
+                                              ix->del_slots, uint32_t(k), uint32_t(n - k), ctx->ws.status);
+        const cudaError_t e = cudaGetLastError();
+        st = e != cudaSuccess ? cuda_fail(ctx, e, "ix_update_kernel") : await_status(ctx, &bits);
+    }
+    if (st != RZ_OK || bits != 0) {
+        // Nothing moved (or the device gave up): the index keeps its keys. The update has looked at
+        // the status by the time the stream is idle.
+        ix_unclaim_kernel<<<grid, 256, 0, s>>>(ix->claims, ix->del_slots, uint32_t(k));
+        cudaStreamSynchronize(s);
+        cudaMemset(ctx->ws.status, 0, sizeof(uint32_t));
+        ctx->ws.dirty = true;
+        return st != RZ_OK ? st : map_status(bits);
+    }
     if (flags & RZ_SYNC) RZ_CUDA_TRY(ctx, cudaStreamSynchronize(s));
     return RZ_OK;
 }

@@ -232,7 +232,7 @@ int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
     if (st != RZ_OK) return st;
     const bool validate = (flags & RZ_VALIDATE) != 0;
     int launches = 0;
-    if (validate) {
+    if (validate && !(flags & kPrevalidated)) {
         st = launch_validate(ctx, n, idx, k, s);
         if (st != RZ_OK) return st;
         launches += 2;

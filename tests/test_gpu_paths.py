@@ -132,3 +132,48 @@ def test_partition_runs_of_tiles(ctx, words, n_tiles, extra):
         room[1:] = on_gpu(host)
         assert ctx.partition(room[1:], d_idx, flags=rz.RZ_SYNC) == n - k
         assert np.array_equal(room[1: n - k + 1].cpu().numpy().view(np.uint32), exp)
+
+
+@pytest.mark.parametrize("words", [2, 4, 8])
+@pytest.mark.parametrize("n,k", [(1, 1), (300, 300), (5000, 257), (70000, 20000)])
+def test_remove_by_key_after_refused_calls(ctx, words, n, k):
+    """rz_remove_by_key after calls that were refused (a key twice, a missing and a reserved key, on
+    the same index): those change neither table nor index and let go of their slots, and the good
+    call that follows gives the oracle's table and an index that is exact; erased keys can be
+    inserted and deleted again."""
+    rng = np.random.default_rng(n * 8 + words)
+    host = payload(n, words, seed=k)
+    keys = rng.permutation(np.arange(1, 2 * n + 1, dtype=np.uint64) * np.uint64(0x9E3779B97F4A7C15))[:n]
+    host[:, :2] = keys.view(np.uint32).reshape(n, 2)
+    table = on_gpu(host)
+    ix = rz.KeyIndex(ctx, 2 * n)
+    ix.build(table)
+    pick = rng.choice(n, size=k, replace=False).astype(np.uint32)
+
+    def dev(a):
+        return torch.from_numpy(a.view(np.int64).copy()).to(DEV)
+
+    wrong = [(np.concatenate([keys[pick[:-1]], np.array([7], np.uint64)]), 3),
+             (np.concatenate([keys[pick[:-1]], np.array([2**64 - 1], np.uint64)]), 3)]
+    if k > 1:
+        wrong.append((np.concatenate([keys[pick[:-1]], keys[pick[:1]]]), 2))
+    for bad, code in wrong:
+        with pytest.raises(rz.RedzoneError) as e:
+            ix.remove_by_key(table, n, dev(bad))
+        assert e.value.code == code
+    assert np.array_equal(table.cpu().numpy().view(np.uint32), host)
+    assert np.array_equal(ix.find(dev(keys)).cpu().numpy(), np.arange(n))
+    assert ix.remove_by_key(table, n, dev(keys[pick])) == n - k
+    exp = host.copy()
+    oracle.remove(exp, pick)
+    got = table.cpu().numpy().view(np.uint32)
+    assert np.array_equal(got[: n - k], exp[: n - k])
+    left = np.ascontiguousarray(exp[: n - k, :2]).view(np.uint64).reshape(-1)
+    if n > k:
+        assert np.array_equal(ix.find(dev(left)).cpu().numpy(), np.arange(n - k))
+    assert (ix.find(dev(keys[pick])).cpu().numpy() == -1).all()
+    table[n - k:] = on_gpu(host)[torch.from_numpy(pick.astype(np.int64)).to(DEV)]
+    ix.insert(table, n - k, k)
+    assert ix.remove_by_key(table, n, dev(keys[pick]), flags=rz.RZ_SYNC) == n - k
+    assert np.array_equal(table.cpu().numpy().view(np.uint32)[: n - k], exp[: n - k])
+    ix.close()
