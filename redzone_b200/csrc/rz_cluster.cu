@@ -162,7 +162,7 @@ __global__ void redzone_cluster_kernel(const ClusterParams p) {
         }
 #pragma unroll
         for (int j = 0; j < IPT; ++j)
-            if (dv[j] && sv[j]) head[rr[j]] = src[j];
+            if (dv[j] && sv[j]) st_item(head + rr[j], src[j]);
 
         uint32_t dmask[IPT], smask[IPT];
         uint32_t* cbuf = s_cnt[tt & 1u];
@@ -239,7 +239,7 @@ __global__ void redzone_cluster_kernel(const ClusterParams p) {
         const uint32_t base2 = min(uint32_t(c2) * tpc, ntiles) * TILE;
         const uint32_t pos = __ldcg(&p.slist[base2 + (jr - s_ps[c2])]);
         const uint32_t dest = __ldcg(&p.dlist[chunk_base + r]);
-        head[dest] = reinterpret_cast<const T*>(p.data)[pos];
+        st_item(head + dest, reinterpret_cast<const T*>(p.data)[pos]);
     }
     RZ_STAMP(p, 4);
 }

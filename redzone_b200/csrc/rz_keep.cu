@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(256) keep_place_kernel(uint8_t* data, uint32_t
         if (r[q] < n) v[q] = ld_sparse(r[q] < m ? S + base + uint64_t(q) * 256 : A + r[q]);
 #pragma unroll
     for (int q = 0; q < kKeepIpt; ++q)
-        if (r[q] < n) A[base + uint64_t(q) * 256] = v[q];
+        if (r[q] < n) st_item(A + base + uint64_t(q) * 256, v[q]);
 }
 
 template <int W>

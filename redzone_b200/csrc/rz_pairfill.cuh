@@ -211,7 +211,7 @@ __device__ __forceinline__ void fill_holes(const PairFillSmem& s, uint32_t R, ui
         if (i >= k || rr[j] >= cut) continue;  // past the list, or a hole needing no fill
         const uint32_t vw = s.mapV()[i >> 5];
         if (!((vw >> lane) & 1u)) {
-            head[rr[j]] = src[j];  // valid source, valid destination
+            st_item(head + rr[j], src[j]);  // valid source, valid destination
             continue;
         }
         const uint32_t below = __popc(vw & ~s.mapP()[i >> 5] & lt);
@@ -231,7 +231,7 @@ __device__ __forceinline__ void fill_holes(const PairFillSmem& s, uint32_t R, ui
             for (uint32_t c = rank - s.spre()[lo]; c > 0u; --c) sw &= sw - 1u;  // drop lower ones
             spos = lo * 32u + uint32_t(__ffs(sw) - 1);
         }
-        head[rr[j]] = tail[spos];
+        st_item(head + rr[j], tail[spos]);
     }
 }
 

@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kPartBlock) partition_move_kernel(
     for (int j = 0; j < IPT; ++j) {
         if (keep[j]) {
             const uint32_t dst = off + s_cnt[j * NW + warp] + __popc(km[j] & lt);
-            A[dst] = s_stage[j * B + threadIdx.x];
+            st_item(A + dst, s_stage[j * B + threadIdx.x]);
         }
     }
     if (my_stamps && threadIdx.x == 0) my_stamps[3] = globaltimer();
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(kMoveBlock, 1) partition_move_ws_kernel(
         for (int j = 0; j < R; ++j) {
             const uint32_t km = __shfl_sync(0xffffffffu, kw, j);
             const uint32_t ej = __shfl_sync(0xffffffffu, excl, j);
-            if ((km >> lane) & 1u) A[dst0 + ej + __popc(km & lt)] = src[j * 32 + lane];
+            if ((km >> lane) & 1u) st_item(A + (dst0 + ej + __popc(km & lt)), src[j * 32 + lane]);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);

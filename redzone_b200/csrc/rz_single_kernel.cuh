@@ -381,10 +381,10 @@ __device__ __forceinline__ void redzone_single_body(const SingleParams& p) {
                 if (i >= k || rr[j] >= cut) continue;  // past the list, or a hole needing no fill
                 const uint32_t vw = mapV[i >> 5];
                 if (!((vw >> lane) & 1u)) {
-                    head[rr[j]] = src[j];  // valid source, valid destination
+                    st_item(head + rr[j], src[j]);  // valid source, valid destination
                 } else {
                     const uint32_t rank = dbase + cbuf[j * nw + warp] + __popc(vw & ~mapP[i >> 5] & lt);
-                    if (rank < stot) head[rr[j]] = tail[s_src[rank]];
+                    if (rank < stot) st_item(head + rr[j], tail[s_src[rank]]);
                 }
             }
             if (lane == 0) {  // leave the global red-zone bitmap zero for the next call
@@ -443,7 +443,7 @@ __device__ __forceinline__ void redzone_single_body(const SingleParams& p) {
         if (!single) {
 #pragma unroll
             for (int j = 0; j < IPT; ++j)
-                if (dv[j] && sv[j]) head[rr[j]] = src[j];
+                if (dv[j] && sv[j]) st_item(head + rr[j], src[j]);
         }
 
         uint32_t dmask[IPT], smask[IPT];
@@ -510,7 +510,7 @@ __device__ __forceinline__ void redzone_single_body(const SingleParams& p) {
     if (single) {
 #pragma unroll
         for (int j = 0; j < IPT; ++j)
-            if (dv[j] && sv[j]) head[rr[j]] = src[j];
+            if (dv[j] && sv[j]) st_item(head + rr[j], src[j]);
         if (lane == 0) {
 #pragma unroll
             for (int j = 0; j < IPT; ++j) {
@@ -571,9 +571,9 @@ __device__ __forceinline__ void redzone_single_body(const SingleParams& p) {
         const uint32_t ent = __ldcg(&p.slist[base2 + (jr - s_ps[c2])]);
         const uint32_t dest = __ldcg(&p.dlist[chunk_base + r]);
         if constexpr (W == 4) {
-            head[dest] = T(ent);
+            st_item(head + dest, T(ent));
         } else {
-            head[dest] = reinterpret_cast<const T*>(p.data)[ent];
+            st_item(head + dest, reinterpret_cast<const T*>(p.data)[ent]);
         }
     }
     RZ_STAMP(p, 4);
