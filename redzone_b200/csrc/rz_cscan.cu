@@ -76,13 +76,6 @@ __device__ __forceinline__ void cluster_wait() {
         if (p.stamps && threadIdx.x == 0) st_[slot] = globaltimer(); \
     } while (0)
 
-__device__ __forceinline__ uint4 ldg_nc_v4(const uint32_t* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p));
-    return v;
-}
 // Component c of v (c is a constant after unrolling).
 __device__ __forceinline__ uint32_t lane_of(const uint4& v, int c) {
     return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w;
@@ -102,26 +95,6 @@ __global__ void __launch_bounds__(MAXB, 1) redzone_cscan_kernel(const CscanParam
     const uint32_t n = p.n, k = p.k, cut = n - k;
     const int B = blockDim.x, nw = B >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t q = cluster.block_rank();
-
-    // ---- the critical path starts with this CTA's slice of the index list: issue it first ------
-    // Slices are multiples of 4 entries (16-byte aligned); warp w of CTA q reads entries
-    // [sb + w * 1024, +1024), lane l the four at +128 j + 4 l of round j.
-    const uint32_t SL = ((k + kCscanQ - 1) / kCscanQ + 3u) & ~3u;
-    const uint32_t sb = min(q * SL, k), se = min(sb + SL, k);
-    const uint32_t wbase = sb + uint32_t(warp) * kCscanWarpSpan;
-    uint4 sv[kCscanVec];
-#pragma unroll
-    for (int j = 0; j < kCscanVec; ++j) {
-        const uint32_t e = wbase + uint32_t(j) * 128u + uint32_t(lane) * 4u;
-        if (e + 4u <= se) {
-            sv[j] = ldg_nc_v4(p.idx + e);
-        } else {
-            sv[j].x = e < se ? __ldg(p.idx + e) : 0u;
-            sv[j].y = e + 1u < se ? __ldg(p.idx + e + 1u) : 0u;
-            sv[j].z = e + 2u < se ? __ldg(p.idx + e + 2u) : 0u;
-            sv[j].w = 0u;  // e + 3 >= se here
-        }
-    }
 
     T* __restrict__ head = reinterpret_cast<T*>(p.data);
     const T* __restrict__ tail = reinterpret_cast<const T*>(p.data) + cut;
@@ -147,6 +120,36 @@ __global__ void __launch_bounds__(MAXB, 1) redzone_cscan_kernel(const CscanParam
     __shared__ uint32_t s_total;
     __shared__ int s_abort;
 
+    // The maps are cleared while the kernel ahead in the stream ends.
+    for (uint32_t w = threadIdx.x; w < kw; w += B) {  // the four maps
+        mapV[w] = 0u;
+        mapP[w] = 0u;
+        pV[w] = 0u;
+        pP[w] = 0u;
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+
+    // ---- the critical path starts with this CTA's slice of the index list: issue it first ------
+    // Slices are multiples of 4 entries (16-byte aligned); warp w of CTA q reads entries
+    // [sb + w * 1024, +1024), lane l the four at +128 j + 4 l of round j.
+    const uint32_t SL = ((k + kCscanQ - 1) / kCscanQ + 3u) & ~3u;
+    const uint32_t sb = min(q * SL, k), se = min(sb + SL, k);
+    const uint32_t wbase = sb + uint32_t(warp) * kCscanWarpSpan;
+    uint4 sv[kCscanVec];
+#pragma unroll
+    for (int j = 0; j < kCscanVec; ++j) {
+        const uint32_t e = wbase + uint32_t(j) * 128u + uint32_t(lane) * 4u;
+        if (e + 4u <= se) {
+            sv[j] = ld_l2(reinterpret_cast<const uint4*>(p.idx + e));
+        } else {
+            sv[j].x = e < se ? ld_l2(p.idx + e) : 0u;
+            sv[j].y = e + 1u < se ? ld_l2(p.idx + e + 1u) : 0u;
+            sv[j].z = e + 2u < se ? ld_l2(p.idx + e + 2u) : 0u;
+            sv[j].w = 0u;  // e + 3 >= se here
+        }
+    }
+
     if (threadIdx.x == 0) s_abort = p.validate ? ((__ldcg(p.status) & (ST_DUPLICATE | ST_RANGE)) != 0) : 0;
 
     // ---- this CTA's tile: index and tail item (needed only by the final moves) ----------------
@@ -157,15 +160,9 @@ __global__ void __launch_bounds__(MAXB, 1) redzone_cscan_kernel(const CscanParam
         const uint32_t i = chunk_base + uint32_t(j) * B + threadIdx.x;
         rr[j] = 0xffffffffu;
         if (t < ntiles && i < k) {
-            rr[j] = __ldg(&p.idx[i]);
-            src[j] = tail[i];
+            rr[j] = ld_l2(&p.idx[i]);
+            src[j] = ld_l2(tail + i);
         }
-    }
-    for (uint32_t w = threadIdx.x; w < kw; w += B) {  // the four maps
-        mapV[w] = 0u;
-        mapP[w] = 0u;
-        pV[w] = 0u;
-        pP[w] = 0u;
     }
     __syncthreads();  // s_abort, zeroed maps
     if (s_abort) {
@@ -402,14 +399,17 @@ int launch_cscan(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t
     lc.blockDim = dim3(unsigned(block));
     lc.dynamicSmemBytes = smem;
     lc.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = kCscanQ;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr;
     lc.numAttrs = 1;
     if (!cscan_cluster_fits(ctx, f, &lc)) return RZ_ERR_UNSUPPORTED;
+    lc.numAttrs = 2;
     RZ_CUDA_TRY(ctx, cudaLaunchKernelEx(&lc, f, p));
     if (info) {
         info->grid = int(grid);

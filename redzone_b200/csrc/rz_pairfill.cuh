@@ -231,7 +231,7 @@ __device__ __forceinline__ void fill_holes(const PairFillSmem& s, uint32_t R, ui
             for (uint32_t c = rank - s.spre()[lo]; c > 0u; --c) sw &= sw - 1u;  // drop lower ones
             spos = lo * 32u + uint32_t(__ffs(sw) - 1);
         }
-        st_item(head + rr[j], tail[spos]);
+        st_item(head + rr[j], ld_l2(tail + spos));
     }
 }
 

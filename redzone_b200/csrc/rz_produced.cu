@@ -53,7 +53,7 @@ static size_t produced_smem_bytes(uint32_t capacity) {
 
 // Produced lists: k = counts[0], candidates counted in counts[1]. Split schedule (rz_remove with
 // a device index list, see below): k = k_fixed, candidates counted in *cand_count, written by the
-// scan kernel this kernel waits for (pdl); the last CTA to read the count resets it (done).
+// scan kernel this kernel waits for (split); the last CTA to read the count resets it (done).
 struct ProducedParams {
     uint8_t* data;
     const uint32_t* idx;
@@ -65,36 +65,49 @@ struct ProducedParams {
     uint32_t* status;
     unsigned long long* dev_len;
     uint32_t validate;
-    uint32_t pdl;                // wait for the preceding (scan) grid before reading candidates
+    uint32_t split;              // pairing grid of the split schedule: wait for the scan grid before the candidates
     uint32_t full_scan;          // scan-all schedule: every CTA reads the whole (16-byte aligned) list
 };
 
 template <int W, int IPT>
 __global__ void __launch_bounds__(kProducedBlock, 1) redzone_produced_kernel(const ProducedParams p) {
     using T = typename Payload<W>::T;
-    const uint32_t k = p.k_fixed ? p.k_fixed : __ldcg(&p.counts[0]);
-    const uint32_t n = p.n;
-    if (k > p.capacity) {  // uniform: every CTA reads the same counts
-        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(p.status, ST_CAPACITY);
-        return;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0 && p.dev_len) *p.dev_len = (unsigned long long)(n - k);
-    const uint32_t B = blockDim.x, TILE = B * IPT;
-    const uint32_t ntiles = (k + TILE - 1) / TILE;
-    const uint32_t t = blockIdx.x;
-    if (t >= ntiles || k == n) return;  // no tile here, or nothing survives (nothing moves)
-    const uint32_t cut = n - k, kw = (k + 31) >> 5, kwc = (p.capacity + 31) >> 5;
-    const uint32_t chunk_base = t * TILE;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = int(B >> 5);
-    T* __restrict__ head = reinterpret_cast<T*>(p.data);
-    const T* __restrict__ tail = reinterpret_cast<const T*>(p.data) + cut;
-
+    const uint32_t n = p.n, B = blockDim.x, kwc = (p.capacity + 31) >> 5;
     extern __shared__ __align__(16) uint32_t s_dyn[];
     __shared__ uint32_t s_cnt[2][16 * 16 + 1];
     __shared__ uint32_t s_scan[33];
     const PairFillSmem pf{s_dyn, kwc, s_cnt, s_scan};
     uint32_t* mapV = pf.mapV();
     uint32_t* mapP = pf.mapP();
+    auto clear_maps = [&](uint32_t words) {
+        for (uint32_t w = threadIdx.x; w < words; w += B) {
+            mapV[w] = 0u;
+            mapP[w] = 0u;
+        }
+    };
+    // Nothing of the list or its counts is read before the kernel ahead in the stream has ended; the
+    // split schedule's pairing grid reads its tile, which its scan grid leaves alone.
+    if (p.full_scan) clear_maps(kwc);
+    if (!p.split) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
+    const uint32_t k = p.k_fixed ? p.k_fixed : __ldcg(&p.counts[0]);
+    if (k > p.capacity) {  // uniform: every CTA reads the same counts
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(p.status, ST_CAPACITY);
+        return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && p.dev_len) *p.dev_len = (unsigned long long)(n - k);
+    const uint32_t TILE = B * IPT;
+    const uint32_t ntiles = (k + TILE - 1) / TILE;
+    const uint32_t t = blockIdx.x;
+    if (t >= ntiles || k == n) return;  // no tile here, or nothing survives (nothing moves)
+    const uint32_t cut = n - k, kw = (k + 31) >> 5;
+    const uint32_t chunk_base = t * TILE;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = int(B >> 5);
+    T* __restrict__ head = reinterpret_cast<T*>(p.data);
+    const T* __restrict__ tail = reinterpret_cast<const T*>(p.data) + cut;
+
     uint32_t* s_spre = pf.spre();
     uint32_t* s_pos = pf.pos();
     uint32_t* s_val = pf.val();
@@ -115,15 +128,15 @@ __global__ void __launch_bounds__(kProducedBlock, 1) redzone_produced_kernel(con
         rr[j] = 0xffffffffu;
         if (i < k) {
             rr[j] = __ldcg(&p.idx[i]);
-            src[j] = tail[i];
+            src[j] = ld_l2(tail + i);
         }
     }
-    for (uint32_t w = threadIdx.x; w < kw; w += B) {
-        mapV[w] = 0u;
-        mapP[w] = 0u;
-    }
+    if (!p.full_scan) clear_maps(kw);
     // Everything above overlaps the scan grid of the split schedule; the candidates need it done.
-    if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.split) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
     if (threadIdx.x == 0) {
         s_m = __ldcg(p.cand_count);
         if (p.done) {
@@ -328,6 +341,21 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const uint32_t* __restr
     if (__any_sync(0xffffffffu, oor) && lane == 0) atomicOr(status, ST_RANGE);
 }
 
+// The pairing kernel, as a programmatic dependent of whatever kernel is ahead of it in the stream.
+static cudaError_t launch_produced(ProducedFn f, uint32_t grid, size_t smem, cudaStream_t s, const ProducedParams& pp) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(kProducedBlock);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, f, pp);
+}
+
 // Let the pairing kernel for (w, items) use the device's large shared memory; once per device.
 static int allow_produced_smem(rz_ctx* ctx, ProducedFn f, uint32_t w, int items) {
     static std::atomic<uint64_t> done[4][4];
@@ -453,19 +481,9 @@ int launch_split(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t
     pp.status = ctx->ws.status;
     pp.dev_len = ctx->ws.dev_len;
     pp.validate = validate ? 1u : 0u;
-    pp.pdl = 1;
+    pp.split = 1;
     pp.full_scan = 0;
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(grid);
-    lc.blockDim = dim3(kProducedBlock);
-    lc.dynamicSmemBytes = smem;
-    lc.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    RZ_CUDA_TRY(ctx, cudaLaunchKernelEx(&lc, f, pp));
+    RZ_CUDA_TRY(ctx, launch_produced(f, grid, smem, s, pp));
     if (info) {
         info->grid = int(grid);
         info->block = kProducedBlock;
@@ -504,10 +522,9 @@ int launch_scanall(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
     pp.status = ctx->ws.status;
     pp.dev_len = ctx->ws.dev_len;
     pp.validate = validate ? 1u : 0u;
-    pp.pdl = 0;
+    pp.split = 0;
     pp.full_scan = 1;
-    f<<<grid, kProducedBlock, smem, s>>>(pp);
-    RZ_CUDA_TRY(ctx, cudaGetLastError());
+    RZ_CUDA_TRY(ctx, launch_produced(f, grid, smem, s, pp));
     if (info) {
         info->grid = int(grid);
         info->block = kProducedBlock;
@@ -671,10 +688,9 @@ int rz_remove_produced(rz_ctx* ctx, rz_producer* p, void* d_data, uint32_t elem_
     pp.status = ctx->ws.status;
     pp.dev_len = ctx->ws.dev_len;
     pp.validate = validate ? 1u : 0u;
-    pp.pdl = 0;
+    pp.split = 0;
     pp.full_scan = 0;
-    f<<<grid, kProducedBlock, smem, s>>>(pp);
-    RZ_CUDA_TRY(ctx, cudaGetLastError());
+    RZ_CUDA_TRY(ctx, launch_produced(f, grid, smem, s, pp));
     ctx->last_kernels += 1;
     ctx->last_grid = int(grid);
     ctx->last_block = kProducedBlock;

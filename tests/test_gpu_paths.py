@@ -177,3 +177,70 @@ def test_remove_by_key_after_refused_calls(ctx, words, n, k):
     assert ix.remove_by_key(table, n, dev(keys[pick]), flags=rz.RZ_SYNC) == n - k
     assert np.array_equal(table.cpu().numpy().view(np.uint32)[: n - k], exp[: n - k])
     ix.close()
+
+
+@pytest.mark.parametrize("k", [700, 20000])
+def test_capture_after_copies_and_joins(ctx, k):
+    """Removals that may start before the kernel ahead of them has ended, captured behind a copy
+    (rz_append_remove), behind kernels that write their list, and behind a join with another stream;
+    the graph is replayed with other lists and every result is the oracle's."""
+    n, g = 100000, 300
+    rng = np.random.default_rng(k)
+    host, gain = payload(n + g, 2, seed=k), payload(g, 2, seed=k + 1)
+    one = [rng.choice(n + g, size=k, replace=False).astype(np.uint32) for _ in range(3)]
+    two = [rng.choice(n + g - k, size=k, replace=False).astype(np.uint32) for _ in range(3)]
+    start, d, d_gain = on_gpu(host), on_gpu(host), on_gpu(gain)
+    all_one, all_two = on_gpu(np.stack(one)), on_gpu(np.stack(two))
+    idx_one, idx_two = torch.zeros((2, 1, k), dtype=torch.int32, device=DEV)
+    pick = torch.zeros(1, dtype=torch.int64, device=DEV)
+    ctx.append_remove(d, n, d_gain, all_one[0])  # the context's scratch grows outside the capture
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        here = torch.cuda.current_stream()
+        d.copy_(start)
+        torch.index_select(all_one, 0, pick, out=idx_one)
+        ctx.append_remove(d, n, d_gain, idx_one)
+        side.wait_stream(here)
+        with torch.cuda.stream(side):
+            torch.index_select(all_two, 0, pick, out=idx_two)
+        here.wait_stream(side)
+        ctx.remove(d[: n + g - k], idx_two)
+    for q in (0, 2, 1):
+        pick.fill_(q)
+        graph.replay()
+        assert ctx.sync_status() == 0
+        exp = host.copy()
+        exp[n:] = gain
+        oracle.remove(exp, one[q])
+        left = exp[: n + g - k].copy()
+        oracle.remove(left, two[q])
+        assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n + g - 2 * k], left[: n + g - 2 * k])
+
+
+@pytest.mark.parametrize("k", [300, 4096, 9000, 60000])
+def test_back_to_back_removals_on_one_list(ctx, k):
+    """Each call reads what the one before it wrote, with nothing between them (and kernels of other
+    shapes in between): 20 removals from one shrinking list."""
+    n = 1 << 21
+    rng = np.random.default_rng(k)
+    host = payload(n, 1, seed=k)
+    d, exp, m = on_gpu(host), host.copy(), n
+    lists = []
+    for _ in range(20):
+        lists.append(rng.choice(m, size=k, replace=False).astype(np.uint32))
+        m -= k
+    d_lists = [on_gpu(x) for x in lists]
+    torch.cuda.synchronize()
+    m = n
+    for q, x in enumerate(d_lists):
+        ctx.remove(d[:m], x, flags=rz.RZ_FORCE_GRID if q % 7 == 3 else 0)
+        m -= k
+    assert ctx.sync_status() == 0
+    m = n
+    for x in lists:
+        left = exp[:m].copy()
+        oracle.remove(left, x)
+        m -= k
+        exp = left
+    assert np.array_equal(d.cpu().numpy().view(np.uint32)[:m], exp[:m])
