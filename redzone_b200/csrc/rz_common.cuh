@@ -287,6 +287,27 @@ __device__ __forceinline__ u32x8 ld_l2(const u32x8* p) { return u32x8{__ldcg(&p-
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// For kernels with nothing to do before the wait.
+__device__ __forceinline__ void pdl_begin() {
+    pdl_wait();
+    pdl_launch_dependents();
+}
+// Launch f with the attribute (f calls pdl_wait before it touches global memory).
+template <typename... P, typename... A>
+static cudaError_t launch_pdl(void (*f)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(block);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, f, P(args)...);
+}
+
 // ---- scans ------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v) {
     const int lane = threadIdx.x & 31;

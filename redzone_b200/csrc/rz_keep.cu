@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(256) keep_stage_kernel(const uint8_t* __restri
                                                          const uint32_t* __restrict__ keep, uint32_t m,
                                                          uint8_t* __restrict__ stage, uint32_t* status) {
     using T = typename Payload<W>::T;
+    pdl_begin();
     const T* A = reinterpret_cast<const T*>(data);
     T* S = reinterpret_cast<T*>(stage);
     bool oor = false;
@@ -58,7 +59,7 @@ __global__ void __launch_bounds__(256) keep_stage_kernel(const uint8_t* __restri
 #pragma unroll
     for (int q = 0; q < kKeepIpt; ++q) {
         const uint64_t j = base + uint64_t(q) * 256;
-        r[q] = j < m ? __ldg(&keep[j]) : 0xffffffffu;
+        r[q] = j < m ? ld_l2(&keep[j]) : 0xffffffffu;
         oor |= j < m && r[q] >= n;
     }
 #pragma unroll
@@ -76,6 +77,7 @@ template <int W>
 __global__ void __launch_bounds__(256) keep_place_kernel(uint8_t* data, uint32_t n, const uint32_t* __restrict__ keep,
                                                          uint32_t m, const uint8_t* __restrict__ stage) {
     using T = typename Payload<W>::T;
+    pdl_begin();
     T* A = reinterpret_cast<T*>(data);
     const T* S = reinterpret_cast<const T*>(stage);
     const uint64_t base = uint64_t(blockIdx.x) * (256 * kKeepIpt) + threadIdx.x;
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(256) keep_place_kernel(uint8_t* data, uint32_t
 #pragma unroll
     for (int q = 0; q < kKeepIpt; ++q) {
         const uint64_t j = base + uint64_t(q) * 256;
-        r[q] = j < m ? __ldg(&keep[j]) : 0xffffffffu;
+        r[q] = j < m ? ld_l2(&keep[j]) : 0xffffffffu;
     }
 #pragma unroll
     for (int q = 0; q < kKeepIpt; ++q)
@@ -95,25 +97,24 @@ __global__ void __launch_bounds__(256) keep_place_kernel(uint8_t* data, uint32_t
 }
 
 template <int W>
-static void keep_launch(void* data, uint32_t n, const uint32_t* keep, uint32_t m, void* stage, uint32_t* status,
+static cudaError_t keep_launch(void* data, uint32_t n, const uint32_t* keep, uint32_t m, void* stage, uint32_t* status,
                         cudaStream_t s) {
     const uint32_t grid = uint32_t((uint64_t(m) + 256 * kKeepIpt - 1) / (256 * kKeepIpt));
     uint8_t* d = static_cast<uint8_t*>(data);
     uint8_t* st = static_cast<uint8_t*>(stage);
-    keep_stage_kernel<W><<<grid, 256, 0, s>>>(d, n, keep, m, st, status);
-    keep_place_kernel<W><<<grid, 256, 0, s>>>(d, n, keep, m, st);
+    const cudaError_t e = launch_pdl(keep_stage_kernel<W>, grid, 256, 0, s, d, n, keep, m, st, status);
+    return e != cudaSuccess ? e : launch_pdl(keep_place_kernel<W>, grid, 256, 0, s, d, n, keep, m, st);
 }
 
 int launch_keep(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* keep, uint32_t m, void* stage,
                 cudaStream_t s) {
     if (m == 0) return RZ_OK;
     switch (w) {
-        case 4: keep_launch<4>(data, n, keep, m, stage, ctx->ws.status, s); break;
-        case 8: keep_launch<8>(data, n, keep, m, stage, ctx->ws.status, s); break;
-        case 16: keep_launch<16>(data, n, keep, m, stage, ctx->ws.status, s); break;
-        default: keep_launch<32>(data, n, keep, m, stage, ctx->ws.status, s); break;
+        case 4: RZ_CUDA_TRY(ctx, keep_launch<4>(data, n, keep, m, stage, ctx->ws.status, s)); break;
+        case 8: RZ_CUDA_TRY(ctx, keep_launch<8>(data, n, keep, m, stage, ctx->ws.status, s)); break;
+        case 16: RZ_CUDA_TRY(ctx, keep_launch<16>(data, n, keep, m, stage, ctx->ws.status, s)); break;
+        default: RZ_CUDA_TRY(ctx, keep_launch<32>(data, n, keep, m, stage, ctx->ws.status, s)); break;
     }
-    RZ_CUDA_TRY(ctx, cudaGetLastError());
     return RZ_OK;
 }
 

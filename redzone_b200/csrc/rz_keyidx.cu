@@ -52,6 +52,7 @@ __device__ __forceinline__ uint32_t find_slot(const unsigned long long* keys, ui
 
 __global__ void ix_insert_kernel(unsigned long long* keys, uint32_t* rows, uint32_t mask, const uint8_t* data,
                                  uint32_t w, uint32_t first, uint32_t count, uint32_t* status) {
+    pdl_begin();
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
         const uint32_t row = first + q;
         const unsigned long long key = record_key(data, w, row);
@@ -85,6 +86,7 @@ __global__ void ix_insert_kernel(unsigned long long* keys, uint32_t* rows, uint3
 template <typename Row>
 __global__ void ix_find_kernel(const unsigned long long* keys, const uint32_t* rows, uint32_t mask,
                                const unsigned long long* q, uint32_t count, Row* out_rows) {
+    pdl_begin();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const unsigned long long key = q[i];
         const uint32_t s = key >= kErasedKey ? kNoRow : find_slot(keys, mask, key);
@@ -97,6 +99,7 @@ __global__ void ix_find_kernel(const unsigned long long* keys, const uint32_t* r
 __global__ void ix_claim_kernel(const unsigned long long* keys, const uint32_t* rows, uint32_t* claims, uint32_t mask,
                                 const unsigned long long* q, uint32_t count, uint32_t* out_rows, uint32_t* out_slots,
                                 uint32_t* status) {
+    pdl_begin();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const unsigned long long key = q[i];
         const uint32_t s = key >= kErasedKey ? kNoRow : find_slot(keys, mask, key);
@@ -119,6 +122,7 @@ __global__ void ix_claim_kernel(const unsigned long long* keys, const uint32_t* 
 __global__ void ix_update_kernel(unsigned long long* keys, uint32_t* rows, uint32_t* claims, uint32_t mask,
                                  const uint8_t* data, uint32_t w, const uint32_t* holes, const uint32_t* del_slots,
                                  uint32_t count, uint32_t cut, const uint32_t* status) {
+    pdl_begin();
     if (__ldcg(status) != 0u) return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const uint32_t h = holes[i], d = del_slots[i];
@@ -136,8 +140,8 @@ __global__ void ix_unclaim_kernel(uint32_t* claims, const uint32_t* del_slots, u
         if (del_slots[i] != kNoRow) claims[del_slots[i] >> 5] = 0u;
 }
 
-static int grid_for(const rz_ctx* ctx, int64_t count) {
-    return int(std::max<int64_t>(1, std::min<int64_t>(int64_t(ctx->sms) * 8, (count + 255) / 256)));
+static uint32_t grid_for(const rz_ctx* ctx, int64_t count) {
+    return uint32_t(std::max<int64_t>(1, std::min<int64_t>(int64_t(ctx->sms) * 8, (count + 255) / 256)));
 }
 
 }  // namespace rz
@@ -183,9 +187,9 @@ static int ix_find(rz_keyindex* ix, const uint64_t* d_keys, int64_t count, Row* 
     std::lock_guard<std::recursive_mutex> lock(ctx->mu);
     cudaSetDevice(ctx->device);
     if (count == 0) return RZ_OK;
-    ix_find_kernel<<<grid_for(ctx, count), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        ix->keys, ix->rows, ix->mask, reinterpret_cast<const unsigned long long*>(d_keys), uint32_t(count), d_rows);
-    RZ_CUDA_TRY(ctx, cudaGetLastError());
+    RZ_CUDA_TRY(ctx, launch_pdl(ix_find_kernel<Row>, grid_for(ctx, count), 256, 0, reinterpret_cast<cudaStream_t>(stream),
+                                ix->keys, ix->rows, ix->mask, reinterpret_cast<const unsigned long long*>(d_keys),
+                                uint32_t(count), d_rows));
     return RZ_OK;
 }
 
@@ -251,10 +255,9 @@ int rz_keyindex_insert(rz_keyindex* ix, const void* d_data, int64_t first, int64
     cudaSetDevice(ctx->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (count > 0) {
-        ix_insert_kernel<<<grid_for(ctx, count), 256, 0, s>>>(ix->keys, ix->rows, ix->mask,
-                                                              static_cast<const uint8_t*>(d_data), record_bytes,
-                                                              uint32_t(first), uint32_t(count), ix->status);
-        RZ_CUDA_TRY(ctx, cudaGetLastError());
+        RZ_CUDA_TRY(ctx, launch_pdl(ix_insert_kernel, grid_for(ctx, count), 256, 0, s, ix->keys, ix->rows, ix->mask,
+                                    static_cast<const uint8_t*>(d_data), record_bytes, uint32_t(first), uint32_t(count),
+                                    ix->status));
     }
     uint32_t bits = 0;
     const int st = ix_status(ix, s, &bits);
@@ -303,11 +306,10 @@ int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint
     }
     int st = reset_if_dirty(ctx, s);
     if (st != RZ_OK) return st;
-    const int grid = grid_for(ctx, k);
-    ix_claim_kernel<<<grid, 256, 0, s>>>(ix->keys, ix->rows, ix->claims, ix->mask,
-                                         reinterpret_cast<const unsigned long long*>(d_keys), uint32_t(k), ix->del_rows,
-                                         ix->del_slots, ctx->ws.status);
-    RZ_CUDA_TRY(ctx, cudaGetLastError());
+    const uint32_t grid = grid_for(ctx, k);
+    RZ_CUDA_TRY(ctx, launch_pdl(ix_claim_kernel, grid, 256, 0, s, ix->keys, ix->rows, ix->claims, ix->mask,
+                                reinterpret_cast<const unsigned long long*>(d_keys), uint32_t(k), ix->del_rows,
+                                ix->del_slots, ctx->ws.status));
     // The removal, unless the claims failed. A removal that may take the O(n) path knows no such
     // refusal, and the predictor reads the rows: there the host looks at the outcome first.
     const bool look = (flags & (RZ_FORCE_PARTITION | RZ_ALLOW_STABLE | RZ_USE_PREDICTOR)) != 0;
@@ -320,10 +322,9 @@ int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint
     // The status as the removal left it; the index update, which looks at it too, runs meanwhile.
     if (st == RZ_OK && bits == 0) st = queue_status(ctx, s);
     if (st == RZ_OK && bits == 0) {
-        ix_update_kernel<<<grid, 256, 0, s>>>(ix->keys, ix->rows, ix->claims, ix->mask,
-                                              static_cast<const uint8_t*>(d_data), record_bytes, ix->del_rows,
-                                              ix->del_slots, uint32_t(k), uint32_t(n - k), ctx->ws.status);
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_pdl(ix_update_kernel, grid, 256, 0, s, ix->keys, ix->rows, ix->claims, ix->mask,
+                                         static_cast<const uint8_t*>(d_data), record_bytes, ix->del_rows, ix->del_slots,
+                                         uint32_t(k), uint32_t(n - k), ctx->ws.status);
         st = e != cudaSuccess ? cuda_fail(ctx, e, "ix_update_kernel") : await_status(ctx, &bits);
     }
     if (st != RZ_OK || bits != 0) {

@@ -33,6 +33,7 @@ constexpr int kPartMarkLoads = 8;
 template <bool VALIDATE>
 __global__ void __launch_bounds__(256) partition_mark_kernel(const uint32_t* __restrict__ idx, uint32_t k, uint32_t n,
                                                              uint32_t* __restrict__ bits, uint32_t* status) {
+    pdl_begin();
     const uint64_t stride = uint64_t(gridDim.x) * 256 * kPartMarkLoads;
     uint32_t found = 0;
     for (uint64_t b = uint64_t(blockIdx.x) * (256 * kPartMarkLoads) + threadIdx.x; b < k; b += stride) {
@@ -40,7 +41,7 @@ __global__ void __launch_bounds__(256) partition_mark_kernel(const uint32_t* __r
 #pragma unroll
         for (int j = 0; j < kPartMarkLoads; ++j) {
             const uint64_t i = b + uint64_t(j) * 256;
-            r[j] = i < k ? __ldg(&idx[i]) : 0u;
+            r[j] = i < k ? ld_l2(&idx[i]) : 0u;
         }
 #pragma unroll
         for (int j = 0; j < kPartMarkLoads; ++j) {
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(256) partition_count_kernel(const uint32_t* __
     __shared__ uint32_t s_kept[kPartMaxRun + 1];
     __shared__ uint32_t s_scan[33];
     __shared__ uint32_t s_last;
+    pdl_begin();
     const int lane = threadIdx.x & 31;
     const uint32_t t0 = blockIdx.x * run, m = min(run, ntiles - t0);
     for (uint32_t q = threadIdx.x >> 5; q < m; q += 8) {
@@ -88,7 +90,7 @@ __global__ void __launch_bounds__(256) partition_count_kernel(const uint32_t* __
 #pragma unroll
         for (int j = 0; j < V; ++j) {
             const uint32_t u = uint32_t(j) * 32u + uint32_t(lane);
-            v[j] = u < BW / 4 ? __ldg(&src[u]) : make_uint4(0u, 0u, 0u, 0u);
+            v[j] = u < BW / 4 ? ld_l2(&src[u]) : make_uint4(0u, 0u, 0u, 0u);
         }
         uint32_t removed = 0;
 #pragma unroll
@@ -145,6 +147,7 @@ __global__ void __launch_bounds__(kPartBlock) partition_move_kernel(
     __shared__ T s_stage[IPT * B];
     __shared__ uint32_t s_cnt[IPT * NW + 1];
     __shared__ uint32_t s_tile;
+    pdl_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0 && dev_len) *dev_len = new_len;
     const unsigned long long t_start = stamps ? globaltimer() : 0ull;
 
@@ -160,7 +163,7 @@ __global__ void __launch_bounds__(kPartBlock) partition_move_kernel(
         my_stamps[1] = globaltimer();
     }
     const uint32_t base = tile * TILE;
-    const uint32_t off = __ldg(&p.run_recs[tile / run].x) + __ldg(&p.offset[tile]);
+    const uint32_t off = ld_l2(&p.run_recs[tile / run].x) + ld_l2(&p.offset[tile]);
     T v[IPT];
     uint32_t wd[IPT];
 #pragma unroll
@@ -291,9 +294,10 @@ __global__ void __launch_bounds__(kMoveBlock, 1) partition_move_ws_kernel(
         }
         s_abort = 0u;
         fence_mbar_init();
-        if (blockIdx.x == 0 && dev_len) *dev_len = new_len;
     }
     __syncthreads();
+    pdl_begin();
+    if (blockIdx.x == 0 && threadIdx.x == 0 && dev_len) *dev_len = new_len;
 
     if (warp == kMoveGroups * GW) {
         // ---------------- producer ----------------
@@ -494,20 +498,19 @@ int launch_partition(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint
     sc.run_total = reinterpret_cast<uint32_t*>(sc.run_recs + kPartMaxRuns);
     const uint32_t tag = 1u;
     const int mgrid = int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(ctx->sms) * 8, (uint64_t(k) + 255) / 256)));
-    if (validate) partition_mark_kernel<true><<<mgrid, 256, 0, s>>>(idx, k, n, ctx->ws.part_bits, ctx->ws.status);
-    else partition_mark_kernel<false><<<mgrid, 256, 0, s>>>(idx, k, n, ctx->ws.part_bits, ctx->ws.status);
+    RZ_CUDA_TRY(ctx, launch_pdl(validate ? partition_mark_kernel<true> : partition_mark_kernel<false>, uint32_t(mgrid), 256, 0,
+                                s, idx, k, n, ctx->ws.part_bits, ctx->ws.status));
     // Runs of 8 tiles (one per warp) or more, about four blocks per SM; kPartMaxRun * kPartMaxRuns tiles
     // are more than any list has (n < 2^32 items of 32 bytes: 2^22 tiles).
     const uint32_t most = std::max<uint32_t>(uint32_t(ctx->sms) * 4, (ntiles + kPartMaxRun - 1) / kPartMaxRun);
     const uint32_t run = std::max<uint32_t>((ntiles + most - 1) / most, std::min<uint32_t>(8, ntiles));
     const uint32_t cgrid = (ntiles + run - 1) / run;
     uint32_t* bits = ctx->ws.part_bits;
-    switch (w) {
-        case 4: partition_count_kernel<kTileBytes / 4 / 32><<<cgrid, 256, 0, s>>>(bits, n, ntiles, run, sc); break;
-        case 8: partition_count_kernel<kTileBytes / 8 / 32><<<cgrid, 256, 0, s>>>(bits, n, ntiles, run, sc); break;
-        case 16: partition_count_kernel<kTileBytes / 16 / 32><<<cgrid, 256, 0, s>>>(bits, n, ntiles, run, sc); break;
-        default: partition_count_kernel<kTileBytes / 32 / 32><<<cgrid, 256, 0, s>>>(bits, n, ntiles, run, sc); break;
-    }
+    const auto count = w == 4   ? partition_count_kernel<kTileBytes / 4 / 32>
+                       : w == 8 ? partition_count_kernel<kTileBytes / 8 / 32>
+                       : w == 16 ? partition_count_kernel<kTileBytes / 16 / 32>
+                                 : partition_count_kernel<kTileBytes / 32 / 32>;
+    RZ_CUDA_TRY(ctx, launch_pdl(count, cgrid, 256, 0, s, bits, n, ntiles, run, sc));
     const uint64_t dev_bit = 1ull << (ctx->device & 63);  // function attributes belong to a device (first 64)
     int grid = int(ntiles), block = kPartBlock;
     if ((reinterpret_cast<uintptr_t>(data) & 15u) == 0 && !ctx->ws.stamps_on) {
@@ -521,15 +524,15 @@ int launch_partition(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint
         }
         grid = std::max(1, std::min<int>(ctx->sms, int(ntiles)));
         block = kMoveBlock;
-        f<<<grid, kMoveBlock, smem, s>>>(static_cast<uint8_t*>(data), n, ntiles, bits, sc, run, tag, ctx->ws.status,
-                                         kSpinLimit, ctx->ws.dev_len, n - k);
+        RZ_CUDA_TRY(ctx, launch_pdl(f, uint32_t(grid), kMoveBlock, smem, s, static_cast<uint8_t*>(data), n, ntiles, bits, sc,
+                                    run, tag, ctx->ws.status, kSpinLimit, ctx->ws.dev_len, n - k));
     } else {
         const uint32_t stride = std::max<uint32_t>(1u, (ntiles + kMaxGrid - 1) / kMaxGrid);
-        move_fn(int(w))<<<ntiles, kPartBlock, 0, s>>>(
-            static_cast<uint8_t*>(data), n, ntiles, bits, sc, run, tag, ctx->ws.status, kSpinLimit, ctx->ws.dev_len, n - k, ctx->ws.stamps_on ? ctx->ws.stamps : nullptr, stride);
+        RZ_CUDA_TRY(ctx, launch_pdl(move_fn(int(w)), ntiles, kPartBlock, 0, s, static_cast<uint8_t*>(data), n, ntiles, bits, sc,
+                                    run, tag, ctx->ws.status, kSpinLimit, ctx->ws.dev_len, n - k,
+                                    ctx->ws.stamps_on ? ctx->ws.stamps : nullptr, stride));
         grid = std::min<int>(int(ntiles), kMaxGrid);
     }
-    RZ_CUDA_TRY(ctx, cudaGetLastError());
     if (info) {
         info->grid = grid;
         info->block = block;

@@ -341,21 +341,6 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const uint32_t* __restr
     if (__any_sync(0xffffffffu, oor) && lane == 0) atomicOr(status, ST_RANGE);
 }
 
-// The pairing kernel, as a programmatic dependent of whatever kernel is ahead of it in the stream.
-static cudaError_t launch_produced(ProducedFn f, uint32_t grid, size_t smem, cudaStream_t s, const ProducedParams& pp) {
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(grid);
-    lc.blockDim = dim3(kProducedBlock);
-    lc.dynamicSmemBytes = smem;
-    lc.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    return cudaLaunchKernelEx(&lc, f, pp);
-}
-
 // Let the pairing kernel for (w, items) use the device's large shared memory; once per device.
 static int allow_produced_smem(rz_ctx* ctx, ProducedFn f, uint32_t w, int items) {
     static std::atomic<uint64_t> done[4][4];
@@ -389,6 +374,7 @@ __global__ void __launch_bounds__(256) produce_where_less_kernel(const rz_produc
     __shared__ uint32_t s_n, s_base;
     if (threadIdx.x == 0) s_n = 0u;
     __syncthreads();
+    pdl_begin();
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t gtid = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
@@ -423,7 +409,7 @@ __global__ void __launch_bounds__(256) produce_where_less_kernel(const rz_produc
     const uint64_t rest = nstep * kProduceStep, stride = warps * 32u;
     const uint64_t n_round = rest + ((uint64_t(v.n) - rest + 31u) & ~uint64_t(31));
     for (uint64_t i = rest + gtid; i < n_round; i += stride) {
-        const bool take = i < v.n && __ldg(&keys[i]) < threshold;
+        const bool take = i < v.n && ld_l2(&keys[i]) < threshold;
         collect(uint32_t(i), take);
     }
     __syncthreads();
@@ -483,7 +469,7 @@ int launch_split(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t
     pp.validate = validate ? 1u : 0u;
     pp.split = 1;
     pp.full_scan = 0;
-    RZ_CUDA_TRY(ctx, launch_produced(f, grid, smem, s, pp));
+    RZ_CUDA_TRY(ctx, launch_pdl(f, grid, kProducedBlock, smem, s, pp));
     if (info) {
         info->grid = int(grid);
         info->block = kProducedBlock;
@@ -524,7 +510,7 @@ int launch_scanall(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
     pp.validate = validate ? 1u : 0u;
     pp.split = 0;
     pp.full_scan = 1;
-    RZ_CUDA_TRY(ctx, launch_produced(f, grid, smem, s, pp));
+    RZ_CUDA_TRY(ctx, launch_pdl(f, grid, kProducedBlock, smem, s, pp));
     if (info) {
         info->grid = int(grid);
         info->block = kProducedBlock;
@@ -612,8 +598,8 @@ int rz_produce_where_less(rz_producer* p, const uint32_t* d_keys, uint32_t thres
     const uint32_t vec = (reinterpret_cast<uintptr_t>(d_keys) & 15u) == 0 ? 1u : 0u;
     const uint64_t units = vec ? (uint64_t(p->n) / kProduceStep) * 32 + p->n % kProduceStep : uint64_t(p->n);
     const int grid = int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(ctx->sms) * 8, (units + 255) / 256)));
-    produce_where_less_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(v, d_keys, threshold, vec);
-    RZ_CUDA_TRY(ctx, cudaGetLastError());
+    RZ_CUDA_TRY(ctx, launch_pdl(produce_where_less_kernel, uint32_t(grid), 256, 0, reinterpret_cast<cudaStream_t>(stream),
+                                v, d_keys, threshold, vec));
     return RZ_OK;
 }
 
@@ -690,7 +676,7 @@ int rz_remove_produced(rz_ctx* ctx, rz_producer* p, void* d_data, uint32_t elem_
     pp.validate = validate ? 1u : 0u;
     pp.split = 0;
     pp.full_scan = 0;
-    RZ_CUDA_TRY(ctx, launch_produced(f, grid, smem, s, pp));
+    RZ_CUDA_TRY(ctx, launch_pdl(f, grid, kProducedBlock, smem, s, pp));
     ctx->last_kernels += 1;
     ctx->last_grid = int(grid);
     ctx->last_block = kProducedBlock;

@@ -58,6 +58,7 @@ constexpr uint32_t kValidateMapShare = 256;
 template <int LOADS>
 __global__ void __launch_bounds__(256) validate_mark_kernel(const uint32_t* __restrict__ idx, uint32_t k, uint32_t n,
                                                             uint32_t* __restrict__ seen, uint32_t* status) {
+    pdl_begin();
     const uint64_t stride = uint64_t(gridDim.x) * 256 * LOADS;
     uint32_t found = 0;
     for (uint64_t b = uint64_t(blockIdx.x) * (256 * LOADS) + threadIdx.x; b < k; b += stride) {
@@ -65,7 +66,7 @@ __global__ void __launch_bounds__(256) validate_mark_kernel(const uint32_t* __re
 #pragma unroll
         for (int j = 0; j < LOADS; ++j) {
             const uint64_t i = b + uint64_t(j) * 256;
-            r[j] = i < k ? __ldg(&idx[i]) : 0u;
+            r[j] = i < k ? ld_l2(&idx[i]) : 0u;
         }
 #pragma unroll
         for (int j = 0; j < LOADS; ++j) {
@@ -81,10 +82,19 @@ __global__ void __launch_bounds__(256) validate_mark_kernel(const uint32_t* __re
 }
 __global__ void validate_clear_kernel(const uint32_t* __restrict__ idx, uint32_t k, uint32_t n,
                                       uint32_t* __restrict__ seen) {
+    pdl_begin();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) {
-        const uint32_t r = __ldg(&idx[i]);
+        const uint32_t r = ld_l2(&idx[i]);
         if (r < n) seen[r >> 5] = 0u;
     }
+}
+__global__ void __launch_bounds__(256) validate_zero_kernel(uint32_t* __restrict__ seen, uint32_t words) {
+    pdl_begin();
+    const uint32_t quads = words / 4, first = blockIdx.x * 1024u + threadIdx.x;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+        if (first + j * 256u < quads) reinterpret_cast<uint4*>(seen)[first + j * 256u] = make_uint4(0u, 0u, 0u, 0u);
+    if (first < (words & 3u)) seen[4u * quads + first] = 0u;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -207,17 +217,16 @@ int launch_validate(rz_ctx* ctx, uint32_t n, const uint32_t* idx, uint32_t k, cu
     int st = ensure_seen(ctx, n);
     if (st != RZ_OK) return st;
     const uint64_t most = uint64_t(ctx->sms) * kValidateBlocksPerSm, blocks = (uint64_t(k) + 255) / 256;
-    if (blocks <= most)
-        validate_mark_kernel<1><<<std::max(1, int(blocks)), 256, 0, s>>>(idx, k, n, ctx->ws.seen, ctx->ws.status);
-    else
-        validate_mark_kernel<8><<<int(most), 256, 0, s>>>(idx, k, n, ctx->ws.seen, ctx->ws.status);
+    RZ_CUDA_TRY(ctx, launch_pdl(blocks <= most ? validate_mark_kernel<1> : validate_mark_kernel<8>,
+                                uint32_t(std::max<uint64_t>(1, std::min(blocks, most))), 256, 0, s, idx, k, n, ctx->ws.seen,
+                                ctx->ws.status));
     if (uint64_t(n) < uint64_t(kValidateMapShare) * k) {
-        RZ_CUDA_TRY(ctx, cudaMemsetAsync(ctx->ws.seen, 0, (size_t(n) + 31) / 32 * 4, s));
+        const uint32_t words = uint32_t((uint64_t(n) + 31) / 32);
+        RZ_CUDA_TRY(ctx, launch_pdl(validate_zero_kernel, words / 4096 + 1, 256, 0, s, ctx->ws.seen, words));
     } else {
-        const int grid = std::max(1, int(std::min<uint64_t>(uint64_t(ctx->sms) * 4, blocks)));
-        validate_clear_kernel<<<grid, 256, 0, s>>>(idx, k, n, ctx->ws.seen);
+        const uint32_t grid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(ctx->sms) * 4, blocks)));
+        RZ_CUDA_TRY(ctx, launch_pdl(validate_clear_kernel, grid, 256, 0, s, idx, k, n, ctx->ws.seen));
     }
-    RZ_CUDA_TRY(ctx, cudaGetLastError());
     return RZ_OK;
 }
 
