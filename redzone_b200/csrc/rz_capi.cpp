@@ -7,9 +7,19 @@
 #include <cstring>
 #include <new>
 
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
+
 #include "rz_internal.h"
 
 namespace rz {
+
+static inline void cpu_relax() {
+#if defined(__x86_64__)
+    _mm_pause();
+#endif
+}
 
 int cuda_fail(rz_ctx* ctx, cudaError_t e, const char* where) {
     if (ctx) {
@@ -103,10 +113,6 @@ int map_status(uint32_t bits) {
     return RZ_OK;
 }
 
-// The status word (offset 0) and the device length (offset 512) of the workspace block come back
-// in one copy on the call's stream into pinned memory. The caller waits for it by polling an
-// event recorded after the copy, so a synchronous call returns within about a microsecond of
-// the copy landing; after kPollLimit of polling it blocks in cudaEventSynchronize instead.
 static constexpr std::chrono::microseconds kPollLimit{2000};
 
 int wait_event(rz_ctx* ctx, cudaEvent_t ev) {
@@ -127,35 +133,43 @@ int wait_event(rz_ctx* ctx, cudaEvent_t ev) {
     return RZ_OK;
 }
 
-int queue_status(rz_ctx* ctx, cudaStream_t s) {
-    RZ_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->ws.h_result, ctx->ws.status, kResultBytes, cudaMemcpyDeviceToHost, s));
-    RZ_CUDA_TRY(ctx, cudaEventRecord(ctx->done_event, s));
+// A synchronous call's result: a one-warp kernel queued behind the call (report_kernel, rz_single.cu)
+// writes the status word and the device length to pinned host memory, each in an 8-byte word with
+// this report's number in its upper half, and the host watches both words. That replaces a copy and
+// an event query per look (a synchronous call returns SYNC_US sooner); after kPollLimit the host
+// blocks in cudaStreamSynchronize instead.
+int queue_status(rz_ctx* ctx, cudaStream_t s, const uint32_t* status) {
+    ++ctx->report_seq;
+    RZ_CUDA_TRY(ctx, launch_report(status ? status : ctx->ws.status, ctx->ws.dev_len, ctx->ws.d_report, ctx->report_seq, s));
     return RZ_OK;
 }
 
-int await_status(rz_ctx* ctx, uint32_t* status) {
-    const int st = wait_event(ctx, ctx->done_event);
-    if (st != RZ_OK) return st;
-    std::memcpy(status, ctx->ws.h_result, sizeof(uint32_t));
+int await_status(rz_ctx* ctx, cudaStream_t s, uint32_t* status, unsigned long long* len) {
+    const volatile unsigned long long* w = ctx->ws.h_report;
+    const uint32_t seq = ctx->report_seq;
+    auto landed = [&] { return uint32_t(w[0] >> 32) == seq && uint32_t(w[1] >> 32) == seq; };
+    const auto t0 = std::chrono::steady_clock::now();
+    for (uint32_t it = 1; !landed(); ++it) {
+        if ((it & 63u) == 0u && std::chrono::steady_clock::now() - t0 > kPollLimit) {
+            RZ_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+            if (!landed()) return RZ_ERR_CUDA;
+        }
+        cpu_relax();
+    }
+    *status = uint32_t(w[0]);
+    if (len) *len = uint32_t(w[1]);
     return RZ_OK;
 }
 
-int fetch_status(rz_ctx* ctx, cudaStream_t s, uint32_t* status) {
+int fetch_status(rz_ctx* ctx, cudaStream_t s, uint32_t* status, unsigned long long* len) {
     const int st = queue_status(ctx, s);
-    return st != RZ_OK ? st : await_status(ctx, status);
-}
-
-static int fetch_result(rz_ctx* ctx, cudaStream_t s, uint32_t* status, unsigned long long* len) {
-    const int st = fetch_status(ctx, s, status);
-    if (st != RZ_OK) return st;
-    if (len) std::memcpy(len, ctx->ws.h_result + 512, sizeof(unsigned long long));
-    return RZ_OK;
+    return st != RZ_OK ? st : await_status(ctx, s, status, len);
 }
 
 int read_status(rz_ctx* ctx, cudaStream_t s, int64_t* new_len) {
     uint32_t h = 0;
     unsigned long long dl = 0;
-    int st = fetch_result(ctx, s, &h, new_len ? &dl : nullptr);
+    int st = fetch_status(ctx, s, &h, new_len ? &dl : nullptr);
     if (st != RZ_OK) return st;
     if (new_len) *new_len = int64_t(dl);
     if (h) {
@@ -286,22 +300,19 @@ int rz_create(rz_ctx** out, int device) {
     w.arrive64 = reinterpret_cast<unsigned long long*>(b + off_arr64);
     w.stamps = reinterpret_cast<unsigned long long*>(b + off_stamps);
     void* hr = nullptr;
-    e = cudaMallocHost(&hr, kResultBytes);
+    void* dr = nullptr;
+    e = cudaHostAlloc(&hr, 64, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&dr, hr, 0);
     if (e != cudaSuccess) {
         int st = cuda_fail(ctx, e, "pinned result buffer");
+        if (hr) cudaFreeHost(hr);
         cudaFree(p);
         delete ctx;
         return st;
     }
-    w.h_result = static_cast<uint8_t*>(hr);
-    e = cudaEventCreateWithFlags(&ctx->done_event, cudaEventDisableTiming);
-    if (e != cudaSuccess) {
-        int st = cuda_fail(ctx, e, "completion event");
-        cudaFreeHost(hr);
-        cudaFree(p);
-        delete ctx;
-        return st;
-    }
+    std::memset(hr, 0, 64);
+    w.h_report = static_cast<unsigned long long*>(hr);
+    w.d_report = static_cast<unsigned long long*>(dr);
     *out = ctx;
     return RZ_OK;
 }
@@ -312,8 +323,7 @@ void rz_destroy(rz_ctx* ctx) {
     cudaDeviceSynchronize();
     Workspace& w = ctx->ws;
     cudaFree(w.status);
-    if (w.h_result) cudaFreeHost(w.h_result);
-    if (ctx->done_event) cudaEventDestroy(ctx->done_event);
+    if (w.h_report) cudaFreeHost(w.h_report);
     cudaFree(w.bitmap);
     cudaFree(w.dlist);
     cudaFree(w.slist);
@@ -450,7 +460,7 @@ int rz_remove_host_idx(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes
     // Read the device-tracked length back with the status: the step's result crosses to the host.
     unsigned long long dl = 0;
     uint32_t h = 0;
-    st = fetch_result(ctx, s, &h, &dl);
+    st = fetch_status(ctx, s, &h, &dl);
     if (st != RZ_OK) return st;
     if (h) {
         RZ_CUDA_TRY(ctx, cudaMemset(ctx->ws.status, 0, sizeof(uint32_t)));

@@ -54,7 +54,8 @@ struct Workspace {
     uint2* redlist = nullptr;        // red-list schedule: {position, value - cut} per red entry, k
     size_t red_cap = 0;
     unsigned long long* stamps = nullptr;     // optional phase timestamps, 8 per CTA
-    uint8_t* h_result = nullptr;     // pinned host copy of [status .. dev_len] (one D2H per sync)
+    unsigned long long* h_report = nullptr;  // pinned: {report number << 32 | status, number << 32 | length}
+    unsigned long long* d_report = nullptr;  // the same words' device address
     bool stamps_on = false;
     bool dirty = false;
 };
@@ -76,7 +77,7 @@ struct rz_ctx {
     void* async_pipe = nullptr;  // rz::AsyncPipe*, owned (see rz_async.cpp)
     size_t scratch_held = 0;     // bytes of grown context scratch
     size_t scratch_limit = ~size_t(0);  // rz_set_scratch_limit: growth beyond it -> RZ_ERR_NO_MEMORY
-    cudaEvent_t done_event = nullptr;    // completion of a synchronous call's last copy (polled)
+    uint32_t report_seq = 0;             // number of the last report asked for (queue_status)
 };
 
 namespace rz {
@@ -159,16 +160,15 @@ void batch_config_space(rz_batch_cfg* out);
 // The batched configuration the attached list-mix predictor picks (false without one).
 bool predict_batch_cfg(rz_ctx* ctx, const rz_list_desc* lists, int nlists, uint32_t w, rz_batch_cfg* cfg);
 void release_extras(rz_ctx* ctx);
-// The status word (offset 0) and the device length (offset 512) of the workspace block: one
-// device-to-host copy of this many bytes brings both back.
-constexpr size_t kResultBytes = 512 + sizeof(unsigned long long);
 // Wait for an event: poll (about 2 ms), then block. RZ_OK or RZ_ERR_CUDA.
 int wait_event(rz_ctx* ctx, cudaEvent_t ev);
-// The status word and the device length, copied behind what is queued on the stream (the event is
-// recorded after the copy); wait for that copy; both.
-int queue_status(rz_ctx* ctx, cudaStream_t s);
-int await_status(rz_ctx* ctx, uint32_t* status);
-int fetch_status(rz_ctx* ctx, cudaStream_t s, uint32_t* status);
+// Ask for a report of a status word (default: the context's) and the device length behind what is
+// queued on the stream; wait for the last one asked for; both. One report is out at a time.
+int queue_status(rz_ctx* ctx, cudaStream_t s, const uint32_t* status = nullptr);
+int await_status(rz_ctx* ctx, cudaStream_t s, uint32_t* status, unsigned long long* len = nullptr);
+int fetch_status(rz_ctx* ctx, cudaStream_t s, uint32_t* status, unsigned long long* len = nullptr);
+cudaError_t launch_report(const uint32_t* status, const unsigned long long* len, unsigned long long* out, uint32_t seq,
+                          cudaStream_t s);
 // With RZ_VALIDATE: the list was checked by the library itself, and the status word says how that went.
 constexpr uint32_t kPrevalidated = 1u << 31;
 // rz_remove, which also takes kPrevalidated.

@@ -153,7 +153,6 @@ struct rz_keyindex {
     uint32_t* claims = nullptr;      // one bit per slot, zero between calls
     uint32_t mask = 0;
     uint32_t* status = nullptr;      // device
-    uint32_t* h_status = nullptr;    // pinned
     uint32_t* del_rows = nullptr;    // removal list of the current call
     uint32_t* del_slots = nullptr;
     uint32_t* del_own = nullptr;     // their own allocation, once a removal outgrew the index's
@@ -163,11 +162,9 @@ struct rz_keyindex {
 using namespace rz;
 
 static int ix_status(rz_keyindex* ix, cudaStream_t s, uint32_t* bits) {
-    RZ_CUDA_TRY(ix->ctx, cudaMemcpyAsync(ix->h_status, ix->status, 4, cudaMemcpyDeviceToHost, s));
-    RZ_CUDA_TRY(ix->ctx, cudaEventRecord(ix->ctx->done_event, s));
-    const int st = wait_event(ix->ctx, ix->ctx->done_event);
+    int st = queue_status(ix->ctx, s, ix->status);
+    if (st == RZ_OK) st = await_status(ix->ctx, s, bits);
     if (st != RZ_OK) return st;
-    *bits = *ix->h_status;
     if (*bits) RZ_CUDA_TRY(ix->ctx, cudaMemsetAsync(ix->status, 0, 4, s));
     return RZ_OK;
 }
@@ -225,7 +222,6 @@ int rz_keyindex_create(rz_ctx* ctx, int64_t capacity, rz_keyindex** out) {
         e = cudaMemset(ix->claims, 0, (claim_words + 4) * 4);
     }
     if (e == cudaSuccess) e = cudaMemset(ix->keys, 0xff, cap * 8);
-    if (e == cudaSuccess) e = cudaMallocHost(&ix->h_status, 4);
     if (e != cudaSuccess) {
         const int st = cuda_fail(ctx, e, "rz_keyindex_create");
         cudaFree(ix->keys);
@@ -241,7 +237,6 @@ void rz_keyindex_destroy(rz_keyindex* ix) {
     cudaSetDevice(ix->ctx->device);
     cudaFree(ix->keys);
     cudaFree(ix->del_own);
-    if (ix->h_status) cudaFreeHost(ix->h_status);
     delete ix;
 }
 
@@ -325,7 +320,7 @@ int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint
         const cudaError_t e = launch_pdl(ix_update_kernel, grid, 256, 0, s, ix->keys, ix->rows, ix->claims, ix->mask,
                                          static_cast<const uint8_t*>(d_data), record_bytes, ix->del_rows, ix->del_slots,
                                          uint32_t(k), uint32_t(n - k), ctx->ws.status);
-        st = e != cudaSuccess ? cuda_fail(ctx, e, "ix_update_kernel") : await_status(ctx, &bits);
+        st = e != cudaSuccess ? cuda_fail(ctx, e, "ix_update_kernel") : await_status(ctx, s, &bits);
     }
     if (st != RZ_OK || bits != 0) {
         // Nothing moved (or the device gave up): the index keeps its keys. The update has looked at

@@ -369,6 +369,18 @@ int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
     return RZ_OK;
 }
 
+// The end of a synchronous call (queue_status, rz_capi.cpp).
+__global__ void report_kernel(const uint32_t* status, const unsigned long long* len, unsigned long long* out, uint32_t seq) {
+    pdl_begin();
+    if (threadIdx.x >= 2) return;
+    const uint32_t v = threadIdx.x == 0 ? ld_l2(status) : uint32_t(__ldcg(len));
+    *reinterpret_cast<volatile unsigned long long*>(out + threadIdx.x) = (unsigned long long)seq << 32 | v;
+}
+cudaError_t launch_report(const uint32_t* status, const unsigned long long* len, unsigned long long* out, uint32_t seq,
+                          cudaStream_t s) {
+    return launch_pdl(report_kernel, 1, 32, 0, s, status, len, out, seq);
+}
+
 // An empty kernel: what a launch of a given shape costs between two events with no work in it.
 __global__ void empty_launch_kernel() {}
 
