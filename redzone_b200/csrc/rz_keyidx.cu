@@ -204,17 +204,15 @@ int rz_keyindex_create(rz_ctx* ctx, int64_t capacity, rz_keyindex** out) {
     if (!ix) return RZ_ERR_NO_MEMORY;
     ix->ctx = ctx;
     ix->mask = uint32_t(cap - 1);
-    // One allocation: keys | rows | claims | status | rows and slots of a removal of up to cap / 32 keys
-    // (a longer one gets arrays of its own; 2 % of the index).
-    // The removal list starts on 16 bytes, as the scanning schedules want it.
-    const size_t claim_words = ((cap + 31) / 32 + 3) & ~size_t(3), del = std::max<size_t>(size_t(cap / 32), 1024);
-    const size_t off_claims = (size_t(cap) * 12 + 15) & ~size_t(15);
-    uint8_t* mem = nullptr;
-    cudaError_t e = cudaMalloc(&mem, off_claims + (claim_words + 4 + 2 * del) * 4);
+    // Keys, and in a second allocation: rows | claims | status | rows and slots of a removal of up to
+    // cap / 32 keys (a longer one gets arrays of its own; 2 % of the index). The removal list starts on
+    // 16 bytes, as the scanning schedules want it.
+    const size_t row_words = size_t(cap + 3) & ~size_t(3), claim_words = ((cap + 31) / 32 + 3) & ~size_t(3);
+    const size_t del = std::max<size_t>(size_t(cap / 32), 1024);
+    cudaError_t e = cudaMalloc(&ix->keys, cap * 8);
+    if (e == cudaSuccess) e = cudaMalloc(&ix->rows, (row_words + claim_words + 4 + 2 * del) * 4);
     if (e == cudaSuccess) {
-        ix->keys = reinterpret_cast<unsigned long long*>(mem);
-        ix->rows = reinterpret_cast<uint32_t*>(ix->keys + cap);
-        ix->claims = reinterpret_cast<uint32_t*>(mem + off_claims);
+        ix->claims = ix->rows + row_words;
         ix->status = ix->claims + claim_words;
         ix->del_rows = ix->status + 4;
         ix->del_slots = ix->del_rows + del;
@@ -225,6 +223,7 @@ int rz_keyindex_create(rz_ctx* ctx, int64_t capacity, rz_keyindex** out) {
     if (e != cudaSuccess) {
         const int st = cuda_fail(ctx, e, "rz_keyindex_create");
         cudaFree(ix->keys);
+        cudaFree(ix->rows);
         delete ix;
         return st;
     }
@@ -236,6 +235,7 @@ void rz_keyindex_destroy(rz_keyindex* ix) {
     if (!ix) return;
     cudaSetDevice(ix->ctx->device);
     cudaFree(ix->keys);
+    cudaFree(ix->rows);
     cudaFree(ix->del_own);
     delete ix;
 }
