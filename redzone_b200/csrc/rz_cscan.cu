@@ -38,7 +38,7 @@ namespace rz {
 
 constexpr uint32_t kCscanQ = 8;          // CTAs per cluster (portable size)
 constexpr int kCscanVec = 8;             // 16-byte slice loads per thread: 32 entries
-constexpr uint32_t kCscanWarpSpan = 32u * 4u * kCscanVec;  // slice entries per warp (1024)
+constexpr uint32_t kCscanWarpSpan = 32u * 4u * kCscanVec;  // most slice entries per warp (1024)
 constexpr uint32_t kCscanRegCap = 256;   // red entries one CTA pushes to each cluster member
 constexpr int kCscanMaxBlock = 512;
 
@@ -116,8 +116,6 @@ __global__ void __launch_bounds__(MAXB, 1) redzone_cscan_kernel(const CscanParam
     uint32_t* pP = pV + kw;
     uint2* s_reg = reinterpret_cast<uint2*>(pP + kw);  // push region r: [r * cap, +cap)
     __shared__ uint32_t s_qcnt[kCscanQ];     // pushed: red entries of each rank's slice
-    __shared__ uint32_t s_qc[kCscanQ + 1];   // their prefix
-    __shared__ uint32_t s_total;
     __shared__ int s_abort;
 
     // The maps are cleared while the kernel ahead in the stream ends.
@@ -131,11 +129,13 @@ __global__ void __launch_bounds__(MAXB, 1) redzone_cscan_kernel(const CscanParam
     pdl_launch_dependents();
 
     // ---- the critical path starts with this CTA's slice of the index list: issue it first ------
-    // Slices are multiples of 4 entries (16-byte aligned); warp w of CTA q reads entries
-    // [sb + w * 1024, +1024), lane l the four at +128 j + 4 l of round j.
+    // Slices are multiples of 4 entries (16-byte aligned), spread over all warps in as few rounds of 128
+    // entries as they need (at most kCscanVec): warp w of CTA q reads entries [sb + w * 128 rounds,
+    // +128 rounds), lane l the four at +128 j + 4 l of round j.
     const uint32_t SL = ((k + kCscanQ - 1) / kCscanQ + 3u) & ~3u;
-    const uint32_t sb = min(q * SL, k), se = min(sb + SL, k);
-    const uint32_t wbase = sb + uint32_t(warp) * kCscanWarpSpan;
+    const uint32_t sb = min(q * SL, k), slice_end = min(sb + SL, k);
+    const uint32_t rounds = (SL + 128u * uint32_t(nw) - 1u) / (128u * uint32_t(nw));
+    const uint32_t wbase = sb + uint32_t(warp) * (128u * rounds), se = min(slice_end, wbase + 128u * rounds);
     uint4 sv[kCscanVec];
 #pragma unroll
     for (int j = 0; j < kCscanVec; ++j) {
@@ -195,29 +195,28 @@ __global__ void __launch_bounds__(MAXB, 1) redzone_cscan_kernel(const CscanParam
     const uint32_t wred = __reduce_add_sync(0xffffffffu, uint32_t(__popc(bits)));
     if (lane == 0) s_scan[warp] = wred;
     __syncthreads();
-    if (warp == 0) {
-        const uint32_t x = lane < nw ? s_scan[lane] : 0u;
-        const uint32_t inc = warp_inclusive_scan(x);
-        if (lane < nw) s_scan[lane] = inc - x;
-        if (lane == 31) s_scan[32] = inc;
-    }
-    __syncthreads();
+    // Entries of the warps before this one, and of all: every warp adds the counts up for itself.
+    const uint32_t wx = lane < nw ? s_scan[lane] : 0u;
+    const uint32_t wpre = __reduce_add_sync(0xffffffffu, lane < warp ? wx : 0u);
+    const uint32_t mine = __reduce_add_sync(0xffffffffu, wx);
     cluster_wait();  // phase 0: every CTA of the cluster runs
     // The slice's count goes to every member (an overflowing count sends all of them to the slow
     // path, where the regions are not read).
-    if (threadIdx.x < kCscanQ) *cluster.map_shared_rank(&s_qcnt[q], threadIdx.x) = s_scan[32];
+    if (threadIdx.x < kCscanQ) *cluster.map_shared_rank(&s_qcnt[q], threadIdx.x) = mine;
     // Entries in position order (round j, then lane, then c): a warp scan per round that has any.
     const uint32_t wany = __reduce_or_sync(0xffffffffu, bits);
     if (wany) {
-        uint32_t run = s_scan[warp];
+        uint32_t run = wpre;
 #pragma unroll
         for (int j = 0; j < kCscanVec; ++j) {
             if (((wany >> (4 * j)) & 15u) == 0u) continue;  // warp-uniform
+            // Entries of the lanes before this one, from the three bits of each lane's count (0..4).
             const uint32_t nib = (bits >> (4 * j)) & 15u;
-            const uint32_t x = uint32_t(__popc(nib));
-            const uint32_t inc = warp_inclusive_scan(x);
-            uint32_t r = run + inc - x;
-            run += __shfl_sync(0xffffffffu, inc, 31);
+            const uint32_t x = uint32_t(__popc(nib)), lt = lanemask_lt();
+            const uint32_t b0 = __ballot_sync(0xffffffffu, x & 1u), b1 = __ballot_sync(0xffffffffu, x & 2u),
+                           b2 = __ballot_sync(0xffffffffu, x & 4u);
+            uint32_t r = run + uint32_t(__popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt));
+            run += uint32_t(__popc(b0) + 2 * __popc(b1) + 4 * __popc(b2));
             const uint32_t e0 = wbase + uint32_t(j) * 128u + uint32_t(lane) * 4u;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -240,27 +239,32 @@ __global__ void __launch_bounds__(MAXB, 1) redzone_cscan_kernel(const CscanParam
     CS_STAMP(2);
 
     // ---- the cluster's red entries, from this CTA's own shared memory ---------------------------
-    if (threadIdx.x < 32) {
-        const uint32_t c = uint32_t(lane) < kCscanQ ? s_qcnt[lane] : 0u;
-        const uint32_t inc = warp_inclusive_scan(c);
-        if (uint32_t(lane) < kCscanQ) s_qc[lane] = inc - c;
-        const bool ovf = __any_sync(0xffffffffu, c > kCscanRegCap);
-        if (lane == 31) s_total = (ovf || inc > kFastMaxRed) ? 0xffffffffu : inc;
+    // Every warp prefixes the slices' counts for itself (no block barrier).
+    const uint32_t qc = uint32_t(lane) < kCscanQ ? s_qcnt[lane] : 0u;
+    uint32_t qin = qc;
+#pragma unroll
+    for (int d = 1; d < int(kCscanQ); d <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, qin, d);
+        if (lane >= d) qin += u;
     }
-    __syncthreads();
-    const uint32_t R = s_total;
+    const uint32_t qex = qin - qc, found = __shfl_sync(0xffffffffu, qin, kCscanQ - 1);
+    const uint32_t R = __any_sync(0xffffffffu, qc > kCscanRegCap) || found > kFastMaxRed ? 0xffffffffu : found;
     const bool fast = R <= kFastMaxRed;
     if (fast) {
         cluster_arrive_relaxed();  // phase 2: no remote access from here on
-        for (uint32_t e = threadIdx.x; e < R; e += B) {
+        for (uint32_t e0 = uint32_t(warp) * 32u; e0 < R; e0 += B) {  // whole warps: the shuffles need every lane
+            const uint32_t e = e0 + uint32_t(lane);
             uint32_t r = 0;
 #pragma unroll
-            for (uint32_t u = 1; u < kCscanQ; ++u) r += s_qc[u] <= e ? 1u : 0u;
-            const uint2 en = s_reg[r * kCscanRegCap + (e - s_qc[r])];
-            s_pos[e] = en.x;
-            s_val[e] = en.y;
-            atomicOr(&mapV[en.y >> 5], 1u << (en.y & 31u));
-            atomicOr(&mapP[en.x >> 5], 1u << (en.x & 31u));
+            for (uint32_t u = 1; u < kCscanQ; ++u) r += __shfl_sync(0xffffffffu, qex, int(u)) <= e ? 1u : 0u;
+            const uint32_t at = e - __shfl_sync(0xffffffffu, qex, int(r));
+            if (e < R) {
+                const uint2 en = s_reg[r * kCscanRegCap + at];
+                s_pos[e] = en.x;
+                s_val[e] = en.y;
+                atomicOr(&mapV[en.y >> 5], 1u << (en.y & 31u));
+                atomicOr(&mapP[en.x >> 5], 1u << (en.x & 31u));
+            }
         }
     } else {
         for (uint32_t w = threadIdx.x; w < kw; w += B) {

@@ -90,22 +90,31 @@ __device__ __forceinline__ void derive_pairing(const PairFillSmem& s, uint32_t R
         stot = s.scan[0];
         dbase = s.scan[1];
     } else if (fast) {
-        // Ranks inside this tile: one word of the V \ P map per (round, warp).
-        if (lane == 0) {
+        // Ranks inside this tile: one word of the V \ P map per (round, warp), prefixed by the last warp
+        // before the rounds' barrier when they fit one.
+        if (E <= 32 && warp == nw - 1) {
+            uint32_t x = 0;
+            if (lane < E) {
+                const uint32_t i0 = chunk_base + uint32_t(lane / nw) * B + uint32_t(lane % nw) * 32u;
+                x = (has_tile && i0 < k) ? __popc(mapV[i0 >> 5] & ~mapP[i0 >> 5]) : 0u;
+            }
+            const uint32_t inc = warp_inclusive_scan(x);
+            if (lane < E) cbuf[lane] = inc - x;
+        } else if (E > 32 && lane == 0) {
 #pragma unroll
             for (int j = 0; j < IPT; ++j) {
                 const uint32_t i0 = chunk_base + uint32_t(j) * B + uint32_t(warp) * 32u;
                 cbuf[j * nw + warp] = (has_tile && i0 < k) ? __popc(mapV[i0 >> 5] & ~mapP[i0 >> 5]) : 0u;
             }
         }
-        // Source orphans compacted in position order; destination orphans before this tile and
-        // in all: rounds of B red entries, per-warp ballot counts, one barrier per round.
-        uint32_t dall = 0;
-        for (uint32_t q0 = 0, rd = 0; q0 == 0 || q0 < R; q0 += B, ++rd) {
-            uint32_t* wc = s.cnt[0] + 96u * (rd & 1u);
-            const uint32_t e = q0 + threadIdx.x;
-            uint32_t ps = 0;
-            bool sf = false, af = false, df = false;
+        // Source orphans compacted in position order; destination orphans before this tile and in all.
+        // Rounds of B red entries, twice over: the first pass counts per (round, warp), one barrier
+        // shares the counts, the second pass ranks and places (the flags are cheaper to look up again
+        // than a barrier per round).
+        uint32_t* wc = s.cnt[0];  // source | destination before the tile << 8 | destination << 16
+        auto look = [&](uint32_t e, uint32_t& ps, bool& sf, bool& af, bool& df) {
+            ps = 0;
+            sf = af = df = false;
             if (e < R) {
                 ps = s.pos()[e];
                 const uint32_t v = s.val()[e];
@@ -113,28 +122,31 @@ __device__ __forceinline__ void derive_pairing(const PairFillSmem& s, uint32_t R
                 af = !((mapP[v >> 5] >> (v & 31u)) & 1u);
                 df = af && v < chunk_base;
             }
+        };
+        uint32_t ps;
+        bool sf, af, df;
+        for (uint32_t q0 = 0, at = uint32_t(warp); q0 < R; q0 += B, at += uint32_t(nw)) {
+            look(q0 + threadIdx.x, ps, sf, af, df);
             const uint32_t bs = __ballot_sync(0xffffffffu, sf);
             const uint32_t bd = __ballot_sync(0xffffffffu, df);
             const uint32_t ba = __ballot_sync(0xffffffffu, af);
-            if (lane == 0) {
-                wc[warp] = __popc(bs);
-                wc[32 + warp] = __popc(bd);
-                wc[64 + warp] = __popc(ba);
-            }
-            __syncthreads();
-            uint32_t pre = 0, ts = 0;
-            for (int w2 = 0; w2 < nw; ++w2) {
-                const uint32_t x = wc[w2];
-                pre += w2 < warp ? x : 0u;
-                ts += x;
-                dbase += wc[32 + w2];
-                dall += wc[64 + w2];
-            }
+            if (lane == 0) wc[at] = uint32_t(__popc(bs)) | uint32_t(__popc(bd)) << 8 | uint32_t(__popc(ba)) << 16;
+        }
+        __syncthreads();
+        uint32_t dall = 0;
+        for (uint32_t q0 = 0, at = 0; q0 < R; q0 += B, at += uint32_t(nw)) {
+            const uint32_t x = lane < nw ? wc[at + uint32_t(lane)] : 0u;
+            const uint32_t both = __reduce_add_sync(0xffffffffu, (x & 0xffu) | (x & 0xff00u) << 8);
+            const uint32_t pre = __reduce_add_sync(0xffffffffu, lane < warp ? x & 0xffu : 0u);
+            dall += __reduce_add_sync(0xffffffffu, x >> 16);
+            look(q0 + threadIdx.x, ps, sf, af, df);
+            const uint32_t bs = __ballot_sync(0xffffffffu, sf);
             if (sf) s.src()[stot + pre + __popc(bs & lt)] = ps;
-            stot += ts;
+            stot += both & 0xffffu;
+            dbase += both >> 16;
         }
         if (threadIdx.x == 0 && blockIdx.x == 0 && dall != stot) atomicOr(status, ST_INCONSISTENT);
-        if (warp == 0) warp0_scan_counts(cbuf, E, lane);
+        if (E > 32 && warp == 0) warp0_scan_counts(cbuf, E, lane);
         __syncthreads();
     } else {
         // Per-word prefixes of destination (V & ~P) and source (P & ~V) orphans, in word order:
