@@ -53,6 +53,22 @@ def _stream_handle(stream) -> int | None:
     return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
 
+_pycall = _native.load_pycall()
+_pycall_ready = False
+
+
+def _bind_pycall() -> bool:
+    """Show the list-call extension torch's current-stream lookup (once); False if there is none."""
+    global _pycall_ready
+    import torch
+    raw, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if _pycall is not None and raw is not None and dev is not None:
+        torch.cuda.current_device()  # initialises CUDA in torch
+        _pycall.bind(dev, raw)
+        _pycall_ready = True
+    return _pycall_ready
+
+
 class Context:
     """Owns library scratch (bitmap, orphan lists, barrier state) on one device."""
 
@@ -62,12 +78,14 @@ class Context:
         if st != 0:
             raise RedzoneError(st, "rz_create")
         self.handle = h
+        self._addr = h.value
         self.device = device
 
     def close(self):
         if getattr(self, "handle", None):
             _native.lib.rz_destroy(self.handle)
             self.handle = None
+            self._addr = 0
 
     def __del__(self):
         try:
@@ -94,15 +112,23 @@ class Context:
     def scratch_bytes(self) -> int:
         return int(_native.lib.rz_scratch_bytes(self.handle))
 
+    def _list_call(self, name: str, data, idx, flags: int, stream) -> int:
+        """rz_remove and the functions of its signature: the new length, or RedzoneError."""
+        if _pycall_ready or _bind_pycall():
+            r = _pycall.call(_native.LIST_CALLS[name], self._addr, data, idx, flags,
+                             None if stream is None else _stream_handle(stream))
+            if r < 0:
+                self._check(-r, name)
+            return r
+        out = ctypes.c_int64(0)
+        st = getattr(_native.lib, name)(self.handle, data.data_ptr(), int(data.shape[0]), item_bytes(data), idx.data_ptr(),
+                                        int(idx.numel()), ctypes.byref(out), flags, _stream_handle(stream))
+        self._check(st, name)
+        return out.value
+
     def remove(self, data, idx, flags: int = 0, stream=None) -> int:
         """In-place Redzone removal; returns the new length (n - k)."""
-        n, k = int(data.shape[0]), int(idx.numel())
-        out = ctypes.c_int64(0)
-        st = _native.lib.rz_remove(self.handle, ctypes.c_void_p(data.data_ptr()), n, item_bytes(data),
-                                   ctypes.c_void_p(idx.data_ptr()), k, ctypes.byref(out), flags,
-                                   ctypes.c_void_p(_stream_handle(stream)))
-        self._check(st, "rz_remove")
-        return out.value
+        return self._list_call("rz_remove", data, idx, flags, stream)
 
     def remove_cfg(self, data, idx, cfg: LaunchCfg, flags: int = 0, stream=None) -> None:
         n, k = int(data.shape[0]), int(idx.numel())
@@ -125,31 +151,17 @@ class Context:
 
     def keep(self, data, keep, flags: int = 0, stream=None) -> int:
         """Preserve-list compaction: data[0..m) = (old) data[keep[j]], O(m); returns m."""
-        n, m = int(data.shape[0]), int(keep.numel())
-        out = ctypes.c_int64(0)
-        st = _native.lib.rz_keep(self.handle, ctypes.c_void_p(data.data_ptr()), n, item_bytes(data),
-                                 ctypes.c_void_p(keep.data_ptr()), m, ctypes.byref(out), flags,
-                                 ctypes.c_void_p(_stream_handle(stream)))
-        self._check(st, "rz_keep")
-        return out.value
+        return self._list_call("rz_keep", data, keep, flags, stream)
 
     def partition(self, data, idx, flags: int = 0, stream=None) -> int:
         """O(n) stable partition comparator (survivors keep their order)."""
-        n, k = int(data.shape[0]), int(idx.numel())
-        out = ctypes.c_int64(0)
-        st = _native.lib.rz_partition(self.handle, ctypes.c_void_p(data.data_ptr()), n, item_bytes(data),
-                                      ctypes.c_void_p(idx.data_ptr()), k, ctypes.byref(out), flags,
-                                      ctypes.c_void_p(_stream_handle(stream)))
-        self._check(st, "rz_partition")
-        return out.value
+        return self._list_call("rz_partition", data, idx, flags, stream)
 
     def remove_host_idx(self, data, h_idx, flags: int = 0, stream=None) -> int:
         """Indices in host memory (numpy or pinned torch CPU tensor); synchronous; returns new length."""
-        n = int(data.shape[0])
         if hasattr(h_idx, "data_ptr"):
-            ptr, k = h_idx.data_ptr(), int(h_idx.numel())
-        else:
-            ptr, k = h_idx.ctypes.data, int(h_idx.size)
+            return self._list_call("rz_remove_host_idx", data, h_idx, flags, stream)
+        n, ptr, k = int(data.shape[0]), h_idx.ctypes.data, int(h_idx.size)
         out = ctypes.c_int64(0)
         st = _native.lib.rz_remove_host_idx(self.handle, ctypes.c_void_p(data.data_ptr()), n, item_bytes(data),
                                             ctypes.c_void_p(ptr), k, ctypes.byref(out), flags,

@@ -5,6 +5,8 @@ There is no fallback: if the native library is absent, importing this module rai
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import re
 from pathlib import Path
 
@@ -187,6 +189,25 @@ _sig("rz_set_batch_predictor", c_i32, [c_vp, c_vp])
 _sig("rz_predict_batch_cfg", c_i32, [c_vp, ctypes.POINTER(ListDesc), c_i32, c_u32, ctypes.POINTER(BatchCfg)])
 _sig("rz_phase_stamps", c_i32, [c_vp, c_i32])
 _sig("rz_read_phase_stamps", c_i32, [c_vp, ctypes.POINTER(c_u64), c_i32, ctypes.POINTER(c_i32)])
+
+
+# The list calls (pycall.c): None when the extension was built for another interpreter or not at all.
+PYCALL_PATH = PKG / "_lib" / "_rzcall.so"
+LIST_CALLS = {name: ctypes.cast(getattr(lib, name), c_vp).value
+              for name in ("rz_remove", "rz_remove_host_idx", "rz_partition", "rz_keep")}
+
+
+def load_pycall():
+    if not PYCALL_PATH.exists():
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("_rzcall", str(PYCALL_PATH))
+    spec = importlib.util.spec_from_file_location("_rzcall", PYCALL_PATH, loader=loader)
+    try:
+        mod = importlib.util.module_from_spec(spec)
+        loader.exec_module(mod)
+    except ImportError:
+        return None
+    return mod
 
 
 def status_string(code: int) -> str:

@@ -11,6 +11,7 @@ import concurrent.futures as cf
 import os
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -20,6 +21,7 @@ OUT_DIR = PKG / "_lib"
 OBJ_DIR = PKG / "_lib" / "obj"
 LIB = OUT_DIR / "libredzone_b200.so"
 E2E = OUT_DIR / "rz_e2e"
+PYCALL = OUT_DIR / "_rzcall.so"
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -67,6 +69,7 @@ def build(verbose: bool = False, quiet: bool = False) -> Path:
         if not quiet:
             print(f"redzone_b200: {LIB.name} up to date ({len(srcs)} sources, none rebuilt)")
         build_e2e_driver(quiet)
+        build_pycall(quiet)
         return LIB
     cmd = [NVCC, *ARCH, "-shared", "-o", str(LIB), *map(str, objs), "-lcuda"]
     res = subprocess.run(cmd, capture_output=True, text=True)
@@ -76,7 +79,25 @@ def build(verbose: bool = False, quiet: bool = False) -> Path:
         print(f"redzone_b200: rebuilt {len(rebuilt)} of {len(srcs)} sources "
               f"({', '.join(rebuilt) if rebuilt else 'objects newer than the library'}); linked {LIB.name}")
     build_e2e_driver(quiet)
+    build_pycall(quiet)
     return LIB
+
+
+def build_pycall(quiet: bool = False) -> Path | None:
+    """The Python extension behind Context's list calls (redzone_b200/pycall.c). Without Python's
+    headers it is left out, and those calls go through ctypes."""
+    src, include = PKG / "pycall.c", Path(sysconfig.get_paths()["include"])
+    if not (include / "Python.h").exists():
+        return None
+    if PYCALL.exists() and PYCALL.stat().st_mtime >= src.stat().st_mtime:
+        return PYCALL
+    cmd = ["gcc", "-O2", "-fPIC", "-shared", str(src), "-o", str(PYCALL), f"-I{include}"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"pycall build failed:\n{res.stdout}\n{res.stderr}")
+    if not quiet:
+        print(f"redzone_b200: built {PYCALL.name}")
+    return PYCALL
 
 
 def build_e2e_driver(quiet: bool = False) -> Path:
