@@ -244,3 +244,26 @@ def test_back_to_back_removals_on_one_list(ctx, k):
         m -= k
         exp = left
     assert np.array_equal(d.cpu().numpy().view(np.uint32)[:m], exp[:m])
+
+
+@pytest.mark.parametrize("words", [1, 4])
+@pytest.mark.parametrize("k,red", [(4100, 0), (4100, 33), (8200, 300), (8200, 1024), (16385, 1025), (20001, 2100),
+                                   (65536, 9000), (65535, 65000), (131072, 1500)])
+def test_cluster_scan_over_red_counts(ctx, words, k, red):
+    """Cluster scan with red entries in every amount its paths divide by (32, one block's threads, 256
+    per slice, 1024 in all, more), spread over the list and crowded in its first slice; slices that
+    end inside a warp's rounds."""
+    n = 4 * k
+    rng = np.random.default_rng(k + red)
+    host = payload(n, words, seed=red)
+    reds = rng.choice(k, size=red, replace=False) + (n - k)
+    holes = rng.choice(n - k, size=k - red, replace=False)
+    for crowded in (False, True):
+        idx = np.concatenate([reds, holes]).astype(np.uint32)
+        if not crowded:
+            rng.shuffle(idx)
+        d = on_gpu(host)
+        assert ctx.remove(d, on_gpu(idx), flags=rz.RZ_SYNC) == n - k
+        exp = host.copy()
+        oracle.remove(exp, idx)
+        assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n - k], exp[: n - k]), crowded
