@@ -69,6 +69,7 @@ typedef enum rz_status {
 #define RZ_SCHED_SPLIT   5  /* a scan grid lists the red entries; the pairing grid (launched as its */
                             /* programmatic dependent) reads them; no wait inside either grid     */
 #define RZ_SCHED_SCANALL 6  /* one grid, every CTA reads the whole list; no wait (short lists)    */
+#define RZ_SCHED_BULK    7  /* 4-byte items: holes grouped by range, stored line by line (large k) */
 
 /* Launch configuration of the single-list kernels (one entry of the 63-point tuning space:
  * block x items x grid scale with the schedule chosen by k, or a cluster-scan, scan-all or split

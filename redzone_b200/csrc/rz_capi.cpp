@@ -75,6 +75,27 @@ int ensure_lists(rz_ctx* ctx, size_t k) {
     return RZ_OK;
 }
 
+int ensure_bulk(rz_ctx* ctx, size_t k, cudaStream_t s) {
+    Workspace& ws = ctx->ws;
+    const size_t ctr = bulk_counter_words(), words = (k + 31) / 32;
+    if (ws.bulk_ctr && words <= ws.bulk_pmap_words && k <= ws.bulk_pairs_cap) return RZ_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return RZ_ERR_UNSUPPORTED;
+    }
+    const std::string before = ctx->last_cuda_error;
+    int st = grow(ctx, ws.bulk_ctr, ws.bulk_ctr_cap, ctr, true);
+    if (st == RZ_OK) st = grow(ctx, ws.bulk_pmap, ws.bulk_pmap_words, words, false);
+    if (st == RZ_OK) st = grow(ctx, ws.bulk_pairs, ws.bulk_pairs_cap, k, false);
+    if (st == RZ_ERR_NO_MEMORY) {
+        cudaGetLastError();  // not an error of this call: the grid schedule needs none of it
+        ctx->last_cuda_error = before;
+        return RZ_ERR_UNSUPPORTED;
+    }
+    return st;
+}
+
 int ensure_seen(rz_ctx* ctx, size_t n) {
     return grow(ctx, ctx->ws.seen, ctx->ws.seen_words, (n + 31) / 32 + 1, true);
 }
@@ -95,6 +116,7 @@ int reset_if_dirty(rz_ctx* ctx, cudaStream_t s) {
     if (w.seen) RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.seen, 0, w.seen_words * 4, s));
     if (w.part_bits) RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.part_bits, 0, w.part_words * 4, s));
     if (w.tile_state) RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.tile_state, 0, 128, s));
+    if (w.bulk_ctr) RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.bulk_ctr, 0, w.bulk_ctr_cap * 4, s));
     RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.epoch, 0, 4, s));
     RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.split_count, 0, 8, s));
     RZ_CUDA_TRY(ctx, cudaMemsetAsync(w.arrive, 0, kMaxGrid * 4, s));
@@ -333,6 +355,9 @@ void rz_destroy(rz_ctx* ctx) {
     cudaFree(w.tile_state);
     cudaFree(w.idx_stage);
     cudaFree(w.keep_stage);
+    cudaFree(w.bulk_ctr);
+    cudaFree(w.bulk_pmap);
+    cudaFree(w.bulk_pairs);
     release_extras(ctx);
     delete ctx;
 }

@@ -53,6 +53,12 @@ struct Workspace {
     unsigned long long* arrive64 = nullptr;   // red-list schedule: tag << 32 | red entries, kMaxGrid
     uint2* redlist = nullptr;        // red-list schedule: {position, value - cut} per red entry, k
     size_t red_cap = 0;
+    uint32_t* bulk_ctr = nullptr;    // bulk schedule: hole counts, gate, bucket offsets and cursors, orphan prefixes
+    size_t bulk_ctr_cap = 0;
+    uint32_t* bulk_pmap = nullptr;   // bulk schedule: k bits, entries that are no hole
+    size_t bulk_pmap_words = 0;
+    uint2* bulk_pairs = nullptr;     // bulk schedule: k (hole, item) pairs by bucket
+    size_t bulk_pairs_cap = 0;
     unsigned long long* stamps = nullptr;     // optional phase timestamps, 8 per CTA
     unsigned long long* h_report = nullptr;  // pinned: {report number << 32 | status, number << 32 | length}
     unsigned long long* d_report = nullptr;  // the same words' device address
@@ -94,6 +100,9 @@ int cuda_fail(rz_ctx* ctx, cudaError_t e, const char* where);
 int ensure_lists(rz_ctx* ctx, size_t k);
 int ensure_seen(rz_ctx* ctx, size_t n);
 int ensure_partition(rz_ctx* ctx, size_t n, size_t ntiles);
+// RZ_ERR_UNSUPPORTED when the bulk schedule's scratch is missing and cannot be had now (scratch limit, no
+// memory, or the stream is being captured): the caller then uses the grid schedule.
+int ensure_bulk(rz_ctx* ctx, size_t k, cudaStream_t s);
 int reset_if_dirty(rz_ctx* ctx, cudaStream_t s);
 
 // Kernel launchers (rz_single.cu).
@@ -106,6 +115,12 @@ struct LaunchInfo {
 int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* idx,
                    uint32_t k, const rz_launch_cfg& cfg, uint32_t flags, cudaStream_t s,
                    LaunchInfo* info);
+// Bulk schedule (rz_bulk.cu): whether it is the default, and its two launches (with ensure_bulk's scratch),
+// before and behind the grid kernel.
+size_t bulk_counter_words();
+bool bulk_wanted(uint32_t n, uint32_t k, uint32_t w);
+int launch_bulk_sample(rz_ctx* ctx, uint32_t n, const uint32_t* idx, uint32_t k, cudaStream_t s);
+int launch_bulk(rz_ctx* ctx, void* data, uint32_t n, const uint32_t* idx, uint32_t k, bool validate, cudaStream_t s);
 int launch_partition(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* idx,
                      uint32_t k, uint32_t flags, cudaStream_t s, LaunchInfo* info);
 // Cluster-scan schedule (rz_cscan.cu); RZ_ERR_UNSUPPORTED when a slice of the index list does not
@@ -130,6 +145,7 @@ int launch_scanall(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
 int launch_cluster(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* idx, uint32_t k,
                    const rz_launch_cfg& cfg, bool validate, cudaStream_t s, LaunchInfo* info);
 int cluster_max_block(int w, int items);
+constexpr uint32_t kBulkMinK = 3u << 22, kBulkMinN = 1u << 27;  // bulk schedule by default from here (rz_bulk.cu)
 constexpr uint32_t kClusterMaxK = 1u << 14;  // RZ_SCHED_AUTO uses the cluster schedule up to here
 // The launch-configuration space in its canonical order (rz_autotune.cpp): 48 grid / cluster
 // points (block x items x grid scale, schedule chosen by k), 8 cluster-scan, 4 scan-all and 3

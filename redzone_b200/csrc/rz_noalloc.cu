@@ -196,6 +196,7 @@ extern "C" int rz_remove_noalloc(void* d_data, int64_t n, uint32_t elem_bytes, c
     p.validate = 0;
     p.redlist = nullptr;  // bitmap schedule only: the fixed scratch array has no red list
     p.arrive64 = nullptr;
+    p.gate = nullptr;
 
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3(unsigned(grid));

@@ -181,7 +181,6 @@ int clamp_cfg(const rz_ctx* ctx, uint32_t k, uint32_t w, rz_launch_cfg* cfg) {
 }
 
 int default_cfg(const rz_ctx* ctx, uint32_t n, uint32_t k, uint32_t w, rz_launch_cfg* cfg) {
-    (void)n;
     cfg->use_partition = 0;
     cfg->schedule = RZ_SCHED_AUTO;
     // Measured on B200 (n = 2^28, L2 flushed): up to k = 2^12 the scan-all schedule (one grid, each
@@ -209,6 +208,7 @@ int default_cfg(const rz_ctx* ctx, uint32_t n, uint32_t k, uint32_t w, rz_launch
         cfg->block = 256; cfg->items = 4; cfg->ctas_per_sm = w >= 16 ? 2 : 1;
     } else {
         cfg->block = 1024; cfg->items = 4; cfg->ctas_per_sm = 2;
+        if (bulk_wanted(n, k, w)) cfg->schedule = RZ_SCHED_BULK;  // the shape is the grid schedule's, its fallback
     }
     return clamp_cfg(ctx, k, w, cfg);
 }
@@ -283,6 +283,21 @@ int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
         if (st != RZ_ERR_UNSUPPORTED) return st;
         sched = RZ_SCHED_GRID;  // k beyond one register pass per slice, or no room for the cluster
     }
+    bool bulk = false;
+    if (sched == RZ_SCHED_BULK) {
+        // The phase stamps are the grid kernel's.
+        if (w == 4 && n > k && !ctx->ws.stamps_on) {
+            st = ensure_bulk(ctx, k, s);
+            if (st != RZ_OK && st != RZ_ERR_UNSUPPORTED) return st;
+            bulk = st == RZ_OK;
+        }
+        if (bulk) {
+            st = launch_bulk_sample(ctx, n, idx, k, s);
+            if (st != RZ_OK) return st;
+            launches += 1;
+        }
+        sched = RZ_SCHED_GRID;
+    }
     if (sched == RZ_SCHED_CLUSTER) {
         LaunchInfo ci;
         ci.launches = launches;
@@ -302,7 +317,7 @@ int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
     size_t dsmem = 0;
     long grid = 1;
     const bool few_red = k <= kFastMaxK || double(k) * double(k) <= double(kFastMaxRed) * double(n);
-    if (sched != RZ_SCHED_BLOCK && k <= kRedlistMaxK && few_red && ctx->ws.redlist && ctx->ws.red_cap > k &&
+    if (!bulk && sched != RZ_SCHED_BLOCK && k <= kRedlistMaxK && few_red && ctx->ws.redlist && ctx->ws.red_cap > k &&
         ntiles > 1) {
         st = allow_redlist_smem(ctx, int(w), cfg.items);
         if (st != RZ_OK) return st;
@@ -346,6 +361,7 @@ int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
     p.validate = validate ? 1u : 0u;
     p.redlist = fast ? ctx->ws.redlist : nullptr;
     p.arrive64 = fast ? ctx->ws.arrive64 : nullptr;
+    p.gate = bulk ? ctx->ws.bulk_ctr : nullptr;
 
     SingleFn f = single_fn(int(w), cfg.items);
     cudaLaunchConfig_t lc{};
@@ -360,6 +376,11 @@ int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
     lc.numAttrs = 1;
     RZ_CUDA_TRY(ctx, cudaLaunchKernelEx(&lc, f, p));
     launches += 1;
+    if (bulk) {
+        st = launch_bulk(ctx, data, n, idx, k, validate, s);
+        if (st != RZ_OK) return st;
+        launches += 4;
+    }
     if (info) {
         info->grid = int(grid);
         info->block = cfg.block;

@@ -27,6 +27,8 @@ struct SingleParams {
     // shared memory it needs): red entries per CTA region and tagged per-CTA entry counts.
     uint2* redlist;
     unsigned long long* arrive64;
+    // Bulk schedule: zero there leaves the list to the bulk kernels behind this one. Nullable.
+    const uint32_t* gate;
 };
 
 // Exclusive scan in place of cbuf[0..E) by warp 0 (E <= 256, a few entries per lane); cbuf[E]
@@ -89,6 +91,8 @@ __device__ __forceinline__ void redzone_single_body(const SingleParams& p) {
         s_abort = p.validate ? ((__ldcg(p.status) & (ST_DUPLICATE | ST_RANGE)) != 0) : 0;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && p.dev_len) *p.dev_len = (unsigned long long)(n - k);
+
+    if (p.gate && __ldcg(p.gate) == 0u) return;  // every CTA reads the same word
 
     uint32_t rr[IPT];
     T src[IPT];

@@ -267,3 +267,113 @@ def test_cluster_scan_over_red_counts(ctx, words, k, red):
         exp = host.copy()
         oracle.remove(exp, idx)
         assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n - k], exp[: n - k]), crowded
+
+
+BULK = rz.LaunchCfg(256, 4, 4, 0, 7)
+
+
+@pytest.mark.parametrize("k,gap", [(1, 2), (33, 5), (4096, 40), (8191, 5), (8192, 64), (8193, 9), (100003, 6),
+                                   (303105, 11), (1 << 20, 17)])
+@pytest.mark.parametrize("dist", ["uniform", "runs", "tail", "most"])
+def test_bulk_schedule(ctx, k, gap, dist):
+    """The bulk schedule at the edges of its tiles and buckets: spread holes, runs of 256, holes in one
+    part of the list (done by the grid kernel), nearly all entries red; index lists off 16 bytes; with
+    validation, and twice in a row on one context."""
+    n = k * gap + 7
+    rng = np.random.default_rng(k + gap)
+    if dist == "uniform":
+        idx = rng.permutation(n)[:k]
+    elif dist == "runs":
+        starts = rng.permutation(n // 256 + 1)[: k // 256 + 1]
+        idx = (starts[:, None] * 256 + np.arange(256)).ravel()
+        idx = np.concatenate([idx[idx < n], np.setdiff1d(np.arange(n), idx)])[:k]
+        rng.shuffle(idx)
+    elif dist == "tail":
+        idx = n - 1 - rng.permutation(min(n, 2 * k))[:k]
+    else:
+        idx = np.concatenate([np.arange(n - k, n - k // 8), rng.permutation(n - k)[: k // 8]])
+        rng.shuffle(idx)
+    idx = idx.astype(np.uint32)
+    host = payload(n, 1, seed=k)
+    exp = host.copy()
+    oracle.remove(exp, idx)
+    room = on_gpu(np.concatenate([np.zeros(1, np.uint32), idx]))
+    for d_idx, flags in ((room[1:], 0), (on_gpu(idx), rz.RZ_VALIDATE)):
+        d = on_gpu(host)
+        ctx.remove_cfg(d, d_idx, BULK, flags=flags | rz.RZ_SYNC)
+        assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n - k], exp[: n - k]), flags
+
+
+def test_bulk_schedule_refusals_limits_and_capture():
+    """A list that fails validation changes nothing and the next call is exact; without its scratch
+    memory, and in a capture that finds none, the grid schedule runs instead; a capture that finds
+    the scratch replays the bulk schedule on other lists."""
+    n, k = 400001, 20011
+    rng = np.random.default_rng(3)
+    host = payload(n, 1, seed=3)
+    lists = [rng.permutation(n)[:k].astype(np.uint32) for _ in range(3)]
+    exps = []
+    for idx in lists:
+        exps.append(host.copy())
+        oracle.remove(exps[-1], idx)
+    c = rz.Context(0)
+    start, d, d_idx = on_gpu(host), on_gpu(host), on_gpu(lists[0])
+
+    def check(q):
+        assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n - k], exps[q][: n - k])
+
+    def capture():
+        graph = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            d.copy_(start)
+            c.remove_cfg(d, d_idx, BULK)
+        return graph, c.last_launch()[0]
+
+    c.remove_cfg(d, d_idx, rz.LaunchCfg(256, 4, 4, 0, 3), flags=rz.RZ_SYNC)
+    check(0)
+    c.set_scratch_limit(0)
+    d.copy_(start)
+    c.remove_cfg(d, d_idx, BULK, flags=rz.RZ_SYNC)
+    assert c.last_launch()[0] == 1
+    check(0)
+    c.set_scratch_limit(None)
+    assert capture()[1] == 1
+    for at, val, code in ((5, None, 2), (k - 1, n + 9, 3)):
+        bad = lists[0].copy()
+        bad[at] = bad[at + 1] if val is None else val
+        d.copy_(start)
+        with pytest.raises(rz.RedzoneError) as e:
+            c.remove_cfg(d, on_gpu(bad), BULK, flags=rz.RZ_VALIDATE | rz.RZ_SYNC)
+        assert e.value.code == code
+        assert torch.equal(d, start)
+    graph, launches = capture()
+    assert launches == 6
+    for q in (1, 2, 0):
+        d_idx.copy_(on_gpu(lists[q]))
+        graph.replay()
+        assert c.sync_status() == 0
+        check(q)
+    c.close()
+
+
+def test_bulk_schedule_is_the_default_for_long_lists(ctx):
+    """Default launch at the first size of the bulk schedule and one item below it, against the grid
+    schedule: 3 * 2^22 of 2^27 int32."""
+    n = 1 << 27
+    g = torch.Generator(device=DEV).manual_seed(5)
+    start = torch.arange(n, dtype=torch.int32, device=DEV).view(-1, 1)
+    idx_all = torch.randperm(n, device=DEV, generator=g)[: 3 << 22].to(torch.int32)
+    for k, bulk in ((3 << 22, True), ((3 << 22) - 1, False)):
+        idx, out = idx_all[:k].contiguous(), []
+        for cfg in (None, rz.LaunchCfg(896, 4, 2, 0, 3)):
+            d = start.clone()
+            if cfg is None:
+                ctx.remove(d, idx, flags=rz.RZ_SYNC)
+                assert (ctx.last_launch()[0] == 6) is bulk
+            else:
+                ctx.remove_cfg(d, idx, cfg, flags=rz.RZ_SYNC)
+            out.append(d[: n - k])
+        assert torch.equal(*out)
+        del out, d
+    torch.cuda.empty_cache()
