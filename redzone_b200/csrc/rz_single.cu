@@ -206,6 +206,12 @@ int default_cfg(const rz_ctx* ctx, uint32_t n, uint32_t k, uint32_t w, rz_launch
         cfg->block = 256; cfg->items = 4; cfg->ctas_per_sm = 2;
     } else if (k <= (1u << 17)) {
         cfg->block = 256; cfg->items = 4; cfg->ctas_per_sm = w >= 16 ? 2 : 1;
+    } else if (k <= 160u << 10 && n / 64u >= k) {
+        // 896 x 4 leaves two thirds of the SMs without a tile. us, 896 / 512 threads, 4- to 16-byte items:
+        // k = 160001 uniform 16.7-18.6 / 14.7-16.8, runs of 256 14.5-18.5 / 12.5-15.9, tail 19.0-20.3 /
+        // 18.8-19.4; from 200003 on lists with many red entries pay more for the wider grid (tail 19.7 / 21.9), as do
+        // lists that are not much longer than the removals (n = 4 k = 2^19: 16.6 / 17.5).
+        cfg->block = 512; cfg->items = 4; cfg->ctas_per_sm = 1;
     } else {
         cfg->block = 1024; cfg->items = 4; cfg->ctas_per_sm = 2;
         if (bulk_wanted(n, k, w)) cfg->schedule = RZ_SCHED_BULK;  // the shape is the grid schedule's, its fallback

@@ -377,3 +377,17 @@ def test_bulk_schedule_is_the_default_for_long_lists(ctx):
         assert torch.equal(*out)
         del out, d
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("words", [1, 4])
+@pytest.mark.parametrize("k,gap", [((1 << 17) + 1, 64), (163840, 64), (163841, 64), (163840, 63)])
+def test_grid_shape_between_2e17_and_160k(ctx, words, k, gap):
+    """Grid schedule with 512-thread CTAs: its first and last k and the next one, and a list too short for it."""
+    n = k * gap
+    host = payload(n, words, seed=k)
+    idx = np.random.default_rng(gap).permutation(n)[:k].astype(np.uint32)
+    d = on_gpu(host)
+    assert ctx.remove(d, on_gpu(idx), flags=rz.RZ_SYNC) == n - k
+    assert ctx.last_launch()[2] == (512 if k <= 163840 and gap == 64 else 896)
+    oracle.remove(host, idx)
+    assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n - k], host[: n - k])
