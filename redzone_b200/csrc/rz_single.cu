@@ -88,13 +88,47 @@ __global__ void validate_clear_kernel(const uint32_t* __restrict__ idx, uint32_t
         if (r < n) seen[r >> 5] = 0u;
     }
 }
-__global__ void __launch_bounds__(256) validate_zero_kernel(uint32_t* __restrict__ seen, uint32_t words) {
+// The bits of one word of the map that lie in the red zone, moved to the red-zone bitmap (bit i there
+// is position cut + i).
+__device__ __forceinline__ void mark_red(uint32_t word, uint32_t at, uint32_t cut, uint32_t* red) {
+    if (at < cut) word &= at + 32u <= cut ? 0u : 0xffffffffu << (cut - at);
+    if (!word) return;
+    if (at < cut) {
+        atomicOr(&red[0], word >> (cut - at));
+        return;
+    }
+    const uint32_t off = at - cut, sh = off & 31u, lo = word << sh, hi = sh ? word >> (32u - sh) : 0u;
+    if (lo) atomicOr(&red[off >> 5], lo);
+    if (hi) atomicOr(&red[(off >> 5) + 1u], hi);
+}
+// A valid list's map holds the red zone's bits, which the removal would mark one by one: they are moved
+// word by word while the map is zeroed (n = 50M, k = 2M from the tail, a call: 83.7 us, 88.2 without).
+__global__ void __launch_bounds__(256) validate_zero_kernel(uint32_t* __restrict__ seen, uint32_t words, uint32_t cut,
+                                                            uint32_t* red, const uint32_t* status) {
     pdl_begin();
     const uint32_t quads = words / 4, first = blockIdx.x * 1024u + threadIdx.x;
+    uint4* q = reinterpret_cast<uint4*>(seen);
+    const bool mark = red && (ld_l2(status) & (ST_DUPLICATE | ST_RANGE)) == 0u;
+    if (mark && (blockIdx.x + 1u) * 4096u > cut / 32u) {
+        uint4 v[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) v[j] = first + j * 256u < quads ? ld_l2(&q[first + j * 256u]) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t at = (first + j * 256u) * 128u;  // below n where any bit is set
+            mark_red(v[j].x, at, cut, red);
+            mark_red(v[j].y, at + 32u, cut, red);
+            mark_red(v[j].z, at + 64u, cut, red);
+            mark_red(v[j].w, at + 96u, cut, red);
+        }
+    }
 #pragma unroll
     for (uint32_t j = 0; j < 4; ++j)
-        if (first + j * 256u < quads) reinterpret_cast<uint4*>(seen)[first + j * 256u] = make_uint4(0u, 0u, 0u, 0u);
-    if (first < (words & 3u)) seen[4u * quads + first] = 0u;
+        if (first + j * 256u < quads) q[first + j * 256u] = make_uint4(0u, 0u, 0u, 0u);
+    if (first < (words & 3u)) {
+        if (mark) mark_red(ld_l2(&seen[4u * quads + first]), (4u * quads + first) * 32u, cut, red);
+        seen[4u * quads + first] = 0u;
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -219,16 +253,19 @@ int default_cfg(const rz_ctx* ctx, uint32_t n, uint32_t k, uint32_t w, rz_launch
     return clamp_cfg(ctx, k, w, cfg);
 }
 
-int launch_validate(rz_ctx* ctx, uint32_t n, const uint32_t* idx, uint32_t k, cudaStream_t s) {
+bool validate_marks(uint32_t n, uint32_t k) { return uint64_t(n) < uint64_t(kValidateMapShare) * k; }
+
+int launch_validate(rz_ctx* ctx, uint32_t n, const uint32_t* idx, uint32_t k, cudaStream_t s, uint32_t* red) {
     int st = ensure_seen(ctx, n);
     if (st != RZ_OK) return st;
     const uint64_t most = uint64_t(ctx->sms) * kValidateBlocksPerSm, blocks = (uint64_t(k) + 255) / 256;
     RZ_CUDA_TRY(ctx, launch_pdl(blocks <= most ? validate_mark_kernel<1> : validate_mark_kernel<8>,
                                 uint32_t(std::max<uint64_t>(1, std::min(blocks, most))), 256, 0, s, idx, k, n, ctx->ws.seen,
                                 ctx->ws.status));
-    if (uint64_t(n) < uint64_t(kValidateMapShare) * k) {
+    if (validate_marks(n, k)) {
         const uint32_t words = uint32_t((uint64_t(n) + 31) / 32);
-        RZ_CUDA_TRY(ctx, launch_pdl(validate_zero_kernel, words / 4096 + 1, 256, 0, s, ctx->ws.seen, words));
+        RZ_CUDA_TRY(ctx, launch_pdl(validate_zero_kernel, words / 4096 + 1, 256, 0, s, ctx->ws.seen, words, n - k, red,
+                                    ctx->ws.status));
     } else {
         const uint32_t grid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(ctx->sms) * 4, blocks)));
         RZ_CUDA_TRY(ctx, launch_pdl(validate_clear_kernel, grid, 256, 0, s, idx, k, n, ctx->ws.seen));
@@ -247,14 +284,17 @@ int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
     if (st != RZ_OK) return st;
     const bool validate = (flags & RZ_VALIDATE) != 0;
     int launches = 0;
-    if (validate && !(flags & kPrevalidated)) {
-        st = launch_validate(ctx, n, idx, k, s);
-        if (st != RZ_OK) return st;
-        launches += 2;
-    }
     int sched = cfg.schedule;
     if (flags & RZ_FORCE_BLOCK) sched = RZ_SCHED_BLOCK;
     if (flags & RZ_FORCE_GRID) sched = RZ_SCHED_GRID;
+    bool marked = false;
+    if (validate && !(flags & kPrevalidated)) {
+        // Beyond kRedlistMaxK these two schedules are the grid kernel's bitmap phases.
+        marked = k > kRedlistMaxK && (sched == RZ_SCHED_AUTO || sched == RZ_SCHED_GRID) && validate_marks(n, k);
+        st = launch_validate(ctx, n, idx, k, s, marked ? ctx->ws.bitmap : nullptr);
+        if (st != RZ_OK) return st;
+        launches += 2;
+    }
     if (sched == RZ_SCHED_AUTO) sched = (k <= kClusterMaxK) ? RZ_SCHED_CLUSTER : RZ_SCHED_GRID;
     if (sched == RZ_SCHED_SCANALL) {
         LaunchInfo ci;
@@ -364,7 +404,7 @@ int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
     p.dev_len = ctx->ws.dev_len;
     p.stamps = ctx->ws.stamps_on ? ctx->ws.stamps : nullptr;
     p.spin_limit = kSpinLimit;
-    p.validate = validate ? 1u : 0u;
+    p.validate = marked ? kMarkedByValidation : validate ? 1u : 0u;
     p.redlist = fast ? ctx->ws.redlist : nullptr;
     p.arrive64 = fast ? ctx->ws.arrive64 : nullptr;
     p.gate = bulk ? ctx->ws.bulk_ctr : nullptr;

@@ -8,6 +8,9 @@
 
 namespace rz {
 
+// SingleParams::validate: the validation has marked the red zone, too.
+constexpr uint32_t kMarkedByValidation = 2;
+
 struct SingleParams {
     uint8_t* data;
     const uint32_t* idx;
@@ -105,7 +108,7 @@ __device__ __forceinline__ void redzone_single_body(const SingleParams& p) {
     // per thread (a mark needs nothing but its own entry; phase B re-reads the indices).
     if (!single && t0 < t1) {
         constexpr uint32_t U = kDeepMarkLoads;
-        const uint32_t hi = min(t1 * TILE, k), step = U * uint32_t(B);
+        const uint32_t hi = p.validate == kMarkedByValidation ? 0u : min(t1 * TILE, k), step = U * uint32_t(B);
         uint32_t b = t0 * TILE + threadIdx.x;
         uint32_t r[U];
 #pragma unroll
@@ -125,7 +128,7 @@ __device__ __forceinline__ void redzone_single_body(const SingleParams& p) {
                     } else {
                         const uint32_t off = r[j] - cut;
                         const uint32_t bit = 1u << (off & 31u);
-                        if (p.validate) {
+                        if (p.validate == 1u) {
                             if (atomicOr(&p.bitmap[off >> 5], bit) & bit) atomicOr(p.status, ST_DUPLICATE);
                         } else {
                             atomicOr(&p.bitmap[off >> 5], bit);
@@ -164,7 +167,7 @@ __device__ __forceinline__ void redzone_single_body(const SingleParams& p) {
                 } else {
                     const uint32_t off = r - cut;
                     const uint32_t bit = 1u << (off & 31u);
-                    if (p.validate) {
+                    if (p.validate == 1u) {
                         if (atomicOr(&p.bitmap[off >> 5], bit) & bit) atomicOr(p.status, ST_DUPLICATE);
                     } else {
                         atomicOr(&p.bitmap[off >> 5], bit);

@@ -391,3 +391,33 @@ def test_grid_shape_between_2e17_and_160k(ctx, words, k, gap):
     assert ctx.last_launch()[2] == (512 if k <= 163840 and gap == 64 else 896)
     oracle.remove(host, idx)
     assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n - k], host[: n - k])
+
+
+@pytest.mark.parametrize("k,cut", [(524289, 0), (524289, 1), (524300, 31), (600000, 32), (524321, 100003), (1048575, 3000017)])
+def test_validation_marks_the_red_zone(ctx, k, cut):
+    """Long validated lists take the red zone's marks from the validation's map: cuts on and off its
+    words, everything removed, removals from the tail alone; also after a list that was refused, with
+    one tile per CTA, and without validation right after."""
+    n = k + cut
+    rng = np.random.default_rng(k)
+    host = payload(n, 2, seed=cut)
+    for tail in (False, True):
+        idx = rng.permutation(n)[:k] if not tail else n - 1 - rng.permutation(min(n, k + k // 3))[:k]
+        idx = idx.astype(np.uint32)
+        exp = host.copy()
+        oracle.remove(exp, idx)
+        for bad_val, code in ((idx[1], 2), (n + 5, 3)):
+            bad = idx.copy()
+            bad[0] = bad_val
+            d = on_gpu(host)
+            with pytest.raises(rz.RedzoneError) as e:
+                ctx.remove(d, on_gpu(bad), flags=rz.RZ_VALIDATE | rz.RZ_SYNC)
+            assert e.value.code == code
+            assert np.array_equal(d.cpu().numpy().view(np.uint32), host)
+        for cfg, flags in ((None, rz.RZ_VALIDATE), (rz.LaunchCfg(512, 8, 2, 0, 3), rz.RZ_VALIDATE), (None, 0)):
+            d = on_gpu(host)
+            if cfg is None:
+                ctx.remove(d, on_gpu(idx), flags=flags | rz.RZ_SYNC)
+            else:
+                ctx.remove_cfg(d, on_gpu(idx), cfg, flags=flags | rz.RZ_SYNC)
+            assert np.array_equal(d.cpu().numpy().view(np.uint32)[:cut], exp[:cut]), (tail, cfg, flags)
