@@ -281,7 +281,7 @@ int rz_noalloc_sync_status(rz_stream_t stream);
 
 /* The configuration rz_remove would choose for (n, k, elem_bytes) without a predictor or tuning
  * table: the scan-all schedule up to k = 2^12, the cluster scan up to 2^17 (where it runs), the
- * grid schedule beyond. */
+ * grid schedule beyond, and the bulk schedule for 4-byte items from k = 3 * 2^22 of n = 2^27. */
 int rz_default_cfg(const rz_ctx* ctx, int64_t n, int64_t k, uint32_t elem_bytes,
                    rz_launch_cfg* cfg);
 

@@ -219,11 +219,11 @@ int default_cfg(const rz_ctx* ctx, uint32_t n, uint32_t k, uint32_t w, rz_launch
     cfg->schedule = RZ_SCHED_AUTO;
     // Measured on B200 (n = 2^28, L2 flushed): up to k = 2^12 the scan-all schedule (one grid, each
     // CTA reads the whole list: 7.9 against 8.5 us per call at k = 2^10); the cluster-scan schedule,
-    // which needs no grid-wide wait, from k = 2^13 to 2^17 (7.2 against 11.1 us per call at
-    // k = 2^16, graph steady state). Where the cluster scan does not run (wider
+    // which needs no grid-wide wait, from k = 2^13 to 2^17 (7.1 against 9.0 us per call at
+    // k = 2^16, graph steady state, list not flushed). Where the cluster scan does not run (wider
     // items at k > 2^16, k > 2^17): the grid schedule with 512-item tiles at 2^15, 1024-item tiles
-    // to 2^17 (64 CTAs at 2^16 -- fewer, fuller CTAs shorten the grid-wide wait), and 4096-item
-    // tiles on two CTAs per SM beyond.
+    // to 2^17 (64 CTAs at 2^16 -- fewer, fuller CTAs shorten the grid-wide wait), 2048-item tiles to
+    // 160k in long lists, and 4096-item tiles on two CTAs per SM beyond.
     if (k <= kScanAllMaxK) {
         cfg->block = 256;
         cfg->items = 1;
