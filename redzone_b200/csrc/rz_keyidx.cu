@@ -8,9 +8,10 @@
 // Removal by key keeps the index exact in O(k): the canonical rule moves an item only into a hole
 // below the cut (every other surviving item keeps its row), so after the removal each hole's new
 // occupant is re-pointed at the hole, and the deleted keys are erased. Nothing is rescanned.
-// The lookup also claims each slot it finds (one bit), which catches a key given twice; a missing or repeated
-// key goes into the context's status word, which the removal (as after RZ_VALIDATE's passes) and the
-// index update look at before they change anything. So the whole call is queued at once and the host
+// The lookup also claims the row of each key (one bit of the map that RZ_VALIDATE uses), which catches a key
+// given twice and two keys of one row; it takes the place of RZ_VALIDATE's passes. What it finds wrong
+// goes into the context's status word, which the removal (as after those passes) and the index
+// update look at before they change anything. So the whole call is queued at once and the host
 // waits for it once. Bound by the random accesses of the probes and by that wait: deleting 65521 of
 // 4.2M 32-byte records by key, inserting as many and looking as many up takes 97 us, and took 165 us
 // with a wait after the lookup, validation passes over the rows, and 64-bit rows made from 32-bit ones
@@ -94,22 +95,22 @@ __global__ void ix_find_kernel(const unsigned long long* keys, const uint32_t* r
     }
 }
 
-// Rows and slots of the keys to delete (kNoRow when absent); every slot is claimed. A missing key
-// is an entry outside the list (ST_RANGE), one given twice a duplicate.
-__global__ void ix_claim_kernel(const unsigned long long* keys, const uint32_t* rows, uint32_t* claims, uint32_t mask,
-                                const unsigned long long* q, uint32_t count, uint32_t* out_rows, uint32_t* out_slots,
-                                uint32_t* status) {
+// Rows and slots of the keys to delete (kNoRow when absent); every row is claimed (seen: one bit per
+// row of the list, zero before). A missing key, or one whose row is past the list, is an entry
+// outside it (ST_RANGE); a key given twice, or two keys that lead to one row, a duplicate.
+__global__ void ix_claim_kernel(const unsigned long long* keys, const uint32_t* rows, uint32_t* seen, uint32_t mask,
+                                const unsigned long long* q, uint32_t count, uint32_t n, uint32_t* out_rows,
+                                uint32_t* out_slots, uint32_t* status) {
     pdl_begin();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const unsigned long long key = q[i];
         const uint32_t s = key >= kErasedKey ? kNoRow : find_slot(keys, mask, key);
-        uint32_t row = kNoRow;
-        if (s == kNoRow) {
+        const uint32_t row = s == kNoRow ? kNoRow : rows[s];
+        if (row >= n) {
             atomicOr(status, ST_RANGE);
         } else {
-            row = rows[s];
-            const uint32_t bit = 1u << (s & 31u);
-            if (atomicOr(&claims[s >> 5], bit) & bit) atomicOr(status, ST_DUPLICATE);
+            const uint32_t bit = 1u << (row & 31u);
+            if (atomicOr(&seen[row >> 5], bit) & bit) atomicOr(status, ST_DUPLICATE);
         }
         out_rows[i] = row;
         out_slots[i] = s;
@@ -119,7 +120,7 @@ __global__ void ix_claim_kernel(const unsigned long long* keys, const uint32_t* 
 // After the removal, if it took place: erase the deleted keys, and point the key of the item that
 // moved into each hole below the cut at the hole (a live key, so its probe never ends at a slot
 // that is erased meanwhile).
-__global__ void ix_update_kernel(unsigned long long* keys, uint32_t* rows, uint32_t* claims, uint32_t mask,
+__global__ void ix_update_kernel(unsigned long long* keys, uint32_t* rows, uint32_t* seen, uint32_t mask,
                                  const uint8_t* data, uint32_t w, const uint32_t* holes, const uint32_t* del_slots,
                                  uint32_t count, uint32_t cut, const uint32_t* status) {
     pdl_begin();
@@ -127,17 +128,17 @@ __global__ void ix_update_kernel(unsigned long long* keys, uint32_t* rows, uint3
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const uint32_t h = holes[i], d = del_slots[i];
         keys[d] = kErasedKey;
-        claims[d >> 5] = 0u;  // every claim in the word is this call's
+        seen[h >> 5] = 0u;  // every claim in the word is this call's
         if (h >= cut) continue;
         const uint32_t s = find_slot(keys, mask, record_key(data, w, h));
         if (s != kNoRow) rows[s] = h;
     }
 }
 
-// A removal that did not take place lets go of its slots.
-__global__ void ix_unclaim_kernel(uint32_t* claims, const uint32_t* del_slots, uint32_t count) {
+// A removal that did not take place lets go of its rows.
+__global__ void ix_unclaim_kernel(uint32_t* seen, const uint32_t* del_rows, uint32_t count, uint32_t n) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-        if (del_slots[i] != kNoRow) claims[del_slots[i] >> 5] = 0u;
+        if (del_rows[i] < n) seen[del_rows[i] >> 5] = 0u;
 }
 
 static uint32_t grid_for(const rz_ctx* ctx, int64_t count) {
@@ -150,7 +151,6 @@ struct rz_keyindex {
     rz_ctx* ctx = nullptr;
     unsigned long long* keys = nullptr;
     uint32_t* rows = nullptr;
-    uint32_t* claims = nullptr;      // one bit per slot, zero between calls
     uint32_t mask = 0;
     uint32_t* status = nullptr;      // device
     uint32_t* del_rows = nullptr;    // removal list of the current call
@@ -204,20 +204,19 @@ int rz_keyindex_create(rz_ctx* ctx, int64_t capacity, rz_keyindex** out) {
     if (!ix) return RZ_ERR_NO_MEMORY;
     ix->ctx = ctx;
     ix->mask = uint32_t(cap - 1);
-    // Keys, and in a second allocation: rows | claims | status | rows and slots of a removal of up to
-    // cap / 32 keys (a longer one gets arrays of its own; 2 % of the index). The removal list starts on
-    // 16 bytes, as the scanning schedules want it.
-    const size_t row_words = size_t(cap + 3) & ~size_t(3), claim_words = ((cap + 31) / 32 + 3) & ~size_t(3);
+    // Keys, and in a second allocation: rows | status | rows and slots of a removal of up to cap / 32
+    // keys (a longer one gets arrays of its own; 2 % of the index). The removal list starts on 16
+    // bytes, as the scanning schedules want it.
+    const size_t row_words = size_t(cap + 3) & ~size_t(3);
     const size_t del = std::max<size_t>(size_t(cap / 32), 1024);
     cudaError_t e = cudaMalloc(&ix->keys, cap * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&ix->rows, (row_words + claim_words + 4 + 2 * del) * 4);
+    if (e == cudaSuccess) e = cudaMalloc(&ix->rows, (row_words + 4 + 2 * del) * 4);
     if (e == cudaSuccess) {
-        ix->claims = ix->rows + row_words;
-        ix->status = ix->claims + claim_words;
+        ix->status = ix->rows + row_words;
         ix->del_rows = ix->status + 4;
         ix->del_slots = ix->del_rows + del;
         ix->del_cap = del;
-        e = cudaMemset(ix->claims, 0, (claim_words + 4) * 4);
+        e = cudaMemset(ix->status, 0, 16);
     }
     if (e == cudaSuccess) e = cudaMemset(ix->keys, 0xff, cap * 8);
     if (e != cudaSuccess) {
@@ -299,12 +298,14 @@ int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint
         ix->del_slots = ix->del_own + cap;
         ix->del_cap = cap;
     }
-    int st = reset_if_dirty(ctx, s);
+    int st = ensure_seen(ctx, size_t(n));
+    if (st != RZ_OK) return st;
+    st = reset_if_dirty(ctx, s);
     if (st != RZ_OK) return st;
     const uint32_t grid = grid_for(ctx, k);
-    RZ_CUDA_TRY(ctx, launch_pdl(ix_claim_kernel, grid, 256, 0, s, ix->keys, ix->rows, ix->claims, ix->mask,
-                                reinterpret_cast<const unsigned long long*>(d_keys), uint32_t(k), ix->del_rows,
-                                ix->del_slots, ctx->ws.status));
+    RZ_CUDA_TRY(ctx, launch_pdl(ix_claim_kernel, grid, 256, 0, s, ix->keys, ix->rows, ctx->ws.seen, ix->mask,
+                                reinterpret_cast<const unsigned long long*>(d_keys), uint32_t(k), uint32_t(n),
+                                ix->del_rows, ix->del_slots, ctx->ws.status));
     // The removal, unless the claims failed. A removal that may take the O(n) path knows no such
     // refusal, and the predictor reads the rows: there the host looks at the outcome first.
     const bool look = (flags & (RZ_FORCE_PARTITION | RZ_ALLOW_STABLE | RZ_USE_PREDICTOR)) != 0;
@@ -313,11 +314,11 @@ int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint
     int64_t nl = 0;
     if (st == RZ_OK && bits == 0)
         st = remove_impl(ctx, d_data, n, record_bytes, ix->del_rows, k, &nl,
-                       ((flags & ~kPrevalidated) | RZ_VALIDATE | (look ? 0u : kPrevalidated)) & ~uint32_t(RZ_SYNC), stream);
+                       (flags | RZ_VALIDATE | kPrevalidated) & ~uint32_t(RZ_SYNC), stream);
     // The status as the removal left it; the index update, which looks at it too, runs meanwhile.
     if (st == RZ_OK && bits == 0) st = queue_status(ctx, s);
     if (st == RZ_OK && bits == 0) {
-        const cudaError_t e = launch_pdl(ix_update_kernel, grid, 256, 0, s, ix->keys, ix->rows, ix->claims, ix->mask,
+        const cudaError_t e = launch_pdl(ix_update_kernel, grid, 256, 0, s, ix->keys, ix->rows, ctx->ws.seen, ix->mask,
                                          static_cast<const uint8_t*>(d_data), record_bytes, ix->del_rows, ix->del_slots,
                                          uint32_t(k), uint32_t(n - k), ctx->ws.status);
         st = e != cudaSuccess ? cuda_fail(ctx, e, "ix_update_kernel") : await_status(ctx, s, &bits);
@@ -325,7 +326,7 @@ int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint
     if (st != RZ_OK || bits != 0) {
         // Nothing moved (or the device gave up): the index keeps its keys. The update has looked at
         // the status by the time the stream is idle.
-        ix_unclaim_kernel<<<grid, 256, 0, s>>>(ix->claims, ix->del_slots, uint32_t(k));
+        ix_unclaim_kernel<<<grid, 256, 0, s>>>(ctx->ws.seen, ix->del_rows, uint32_t(k), uint32_t(n));
         cudaStreamSynchronize(s);
         cudaMemset(ctx->ws.status, 0, sizeof(uint32_t));
         ctx->ws.dirty = true;

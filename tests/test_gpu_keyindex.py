@@ -116,3 +116,44 @@ def test_insert_after_append_then_remove_by_key(ctx):
     assert np.array_equal(got[:n], exp[:n])
     assert np.array_equal(ix.find(dev_keys(keys_of(exp[:n]))).cpu().numpy(), np.arange(n))
     ix.close()
+
+
+@pytest.mark.parametrize("k", [2, 33, 3000, 9000, 140000])
+def test_remove_by_key_refuses_rows_past_the_list_and_shared_rows(ctx, k):
+    """Keys whose row is past the n rows of the call (RZ_ERR_OUT_OF_RANGE), and two keys that lead to one
+    row -- a record overwritten in place and indexed again -- (RZ_ERR_DUPLICATE): refused on every
+    schedule with table and index unchanged, and the good call that follows is exact."""
+    n, words = 5 * k + 3, 4
+    host = make_table(n, words, seed=k)
+    d = torch.from_numpy(host.view(np.int32).copy()).to(DEV)
+    ix = rz.KeyIndex(ctx, 4 * n)
+    ix.build(d)
+    rng = np.random.default_rng(k)
+    pick = rng.choice(n - 1, size=k, replace=False)
+    live = keys_of(host)
+
+    def refused(keys, rows, code):
+        with pytest.raises(rz.RedzoneError) as e:
+            ix.remove_by_key(d, rows, dev_keys(keys), flags=rz.RZ_SYNC)
+        assert e.value.code == code
+        assert np.array_equal(d.cpu().numpy().view(np.uint32).reshape(n, words), host)
+        assert np.array_equal(ix.find(dev_keys(live)).cpu().numpy(), np.arange(n))
+
+    past = pick.copy()
+    past[k // 2] = n - 1
+    refused(live[past], n - 1, _native.RZ_ERR_OUT_OF_RANGE)
+    # Row pick[0] gets a new key; the old one stays in the index.
+    old = live[pick[0]]
+    live[pick[0]] = np.uint64(1 << 62)
+    host[pick[0], :2] = [0, 1 << 30]
+    d.copy_(torch.from_numpy(host.view(np.int32)).to(DEV))
+    ix.insert(d, int(pick[0]), 1)
+    shared = live[pick].copy()
+    shared[-1] = old
+    refused(shared, n, _native.RZ_ERR_DUPLICATE)
+    assert ix.remove_by_key(d, n, dev_keys(live[pick]), flags=rz.RZ_SYNC) == n - k
+    exp = host.copy()
+    oracle.remove(exp, pick.astype(np.uint32))
+    assert np.array_equal(d.cpu().numpy().view(np.uint32).reshape(n, words)[: n - k], exp[: n - k])
+    assert np.array_equal(ix.find(dev_keys(keys_of(exp[: n - k]))).cpu().numpy(), np.arange(n - k))
+    ix.close()
