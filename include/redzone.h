@@ -177,9 +177,11 @@ int rz_keep(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, const uin
  *   rz_keyindex_find64 -- the same as 64-bit rows, -1 when absent.
  *   rz_remove_by_key   -- remove the rows holding the k given keys with the Redzone rule and keep
  *                         the index exact: deleted keys are erased and each item moved into a hole
- *                         is re-pointed at it (O(k); no other row changes). Synchronous up to the
- *                         removal: a missing key returns RZ_ERR_OUT_OF_RANGE and a repeated one
- *                         RZ_ERR_DUPLICATE before any row moves. *new_len = n - k.
+ *                         is re-pointed at it (O(k); no other row changes). Synchronous. A missing
+ *                         key, or one whose row is >= n, returns RZ_ERR_OUT_OF_RANGE, and a repeated
+ *                         one, or two of one row, RZ_ERR_DUPLICATE, before any row moves and with or
+ *                         without RZ_VALIDATE. The flags that allow or force the O(n) partition
+ *                         have no effect: its order is not the rule's. *new_len = n - k.
  */
 typedef struct rz_keyindex rz_keyindex;
 int rz_keyindex_create(rz_ctx* ctx, int64_t capacity, rz_keyindex** out);

@@ -288,6 +288,8 @@ int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (new_len) *new_len = n - k;
     if (k == 0) return RZ_OK;
+    // The index follows the Redzone rule only: the O(n) path would move rows that it does not look at.
+    flags &= ~uint32_t(RZ_FORCE_PARTITION | RZ_ALLOW_STABLE);
     if (size_t(k) > ix->del_cap) {
         cudaFree(ix->del_own);
         ix->del_own = ix->del_rows = ix->del_slots = nullptr;
@@ -306,9 +308,9 @@ int rz_remove_by_key(rz_ctx* ctx, rz_keyindex* ix, void* d_data, int64_t n, uint
     RZ_CUDA_TRY(ctx, launch_pdl(ix_claim_kernel, grid, 256, 0, s, ix->keys, ix->rows, ctx->ws.seen, ix->mask,
                                 reinterpret_cast<const unsigned long long*>(d_keys), uint32_t(k), uint32_t(n),
                                 ix->del_rows, ix->del_slots, ctx->ws.status));
-    // The removal, unless the claims failed. A removal that may take the O(n) path knows no such
-    // refusal, and the predictor reads the rows: there the host looks at the outcome first.
-    const bool look = (flags & (RZ_FORCE_PARTITION | RZ_ALLOW_STABLE | RZ_USE_PREDICTOR)) != 0;
+    // The removal, unless the claims failed. The predictor reads the rows: there the host looks at the
+    // outcome first.
+    const bool look = (flags & RZ_USE_PREDICTOR) != 0;
     uint32_t bits = 0;
     if (look) st = fetch_status(ctx, s, &bits);
     int64_t nl = 0;

@@ -1,6 +1,8 @@
 """Delete-by-key through the key -> row index: the table after each removal is the canonical
 result for the rows those keys occupied (checked against the oracle), and the index maps every
 live key to its current row and every deleted key to nothing."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -157,3 +159,27 @@ def test_remove_by_key_refuses_rows_past_the_list_and_shared_rows(ctx, k):
     assert np.array_equal(d.cpu().numpy().view(np.uint32).reshape(n, words)[: n - k], exp[: n - k])
     assert np.array_equal(ix.find(dev_keys(keys_of(exp[: n - k]))).cpu().numpy(), np.arange(n - k))
     ix.close()
+
+
+@pytest.mark.parametrize("flag", [rz.RZ_FORCE_PARTITION, rz.RZ_ALLOW_STABLE, rz.RZ_ALLOW_STABLE | rz.RZ_USE_PREDICTOR,
+                                  rz.RZ_USE_PREDICTOR, rz.RZ_FORCE_GRID, rz.RZ_VALIDATE])
+@pytest.mark.parametrize("k", [5, 3000])
+def test_remove_by_key_follows_the_rule_under_every_flag(flag, k):
+    """Flags that send rz_remove to the order-preserving path, a tuning entry that picks it, and others:
+    the table is the rule's and the index exact."""
+    n, words = 4 * k, 4
+    c = rz.Context(0)
+    cfg = rz.LaunchCfg(256, 4, 2, 1, 0)
+    assert _native.lib.rz_tune_table_set_single(c.handle, words * 4, k.bit_length() - 1, ctypes.byref(cfg)) == 0
+    host = make_table(n, words, seed=k)
+    d = torch.from_numpy(host.view(np.int32).copy()).to(DEV)
+    ix = rz.KeyIndex(c, 2 * n)
+    ix.build(d)
+    pick = np.random.default_rng(k).choice(n, size=k, replace=False)
+    assert ix.remove_by_key(d, n, dev_keys(keys_of(host)[pick]), flags=flag) == n - k
+    exp = host.copy()
+    oracle.remove(exp, pick.astype(np.uint32))
+    assert np.array_equal(d.cpu().numpy().view(np.uint32).reshape(n, words)[: n - k], exp[: n - k])
+    assert np.array_equal(ix.find(dev_keys(keys_of(exp[: n - k]))).cpu().numpy(), np.arange(n - k))
+    ix.close()
+    c.close()
