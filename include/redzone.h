@@ -180,8 +180,10 @@ int rz_keep(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, const uin
  *                         is re-pointed at it (O(k); no other row changes). Synchronous. A missing
  *                         key, or one whose row is >= n, returns RZ_ERR_OUT_OF_RANGE, and a repeated
  *                         one, or two of one row, RZ_ERR_DUPLICATE, before any row moves and with or
- *                         without RZ_VALIDATE. The flags that allow or force the O(n) partition
- *                         have no effect: its order is not the rule's. *new_len = n - k.
+ *                         without RZ_VALIDATE. So does an error that an earlier asynchronous call
+ *                         on the context left unread (that error is returned). The flags that allow
+ *                         or force the O(n) partition have no effect: its order is not the rule's.
+ *                         *new_len = n - k.
  */
 typedef struct rz_keyindex rz_keyindex;
 int rz_keyindex_create(rz_ctx* ctx, int64_t capacity, rz_keyindex** out);

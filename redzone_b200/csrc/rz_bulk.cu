@@ -78,7 +78,7 @@ __device__ __forceinline__ uint32_t bucket_of(const BulkParams& p, uint32_t at) 
 
 // A failed validation leaves the caller's data untouched.
 __device__ __forceinline__ bool bulk_refused(const BulkParams& p) {
-    return p.validate && (__ldcg(p.status) & (ST_DUPLICATE | ST_RANGE)) != 0u;
+    return p.validate && (__ldcg(p.status) & ST_INVALID) != 0u;
 }
 
 __device__ __forceinline__ bool bulk_skip(const BulkParams& p) { return bulk_refused(p) || __ldcg(p.gate) != 0u; }

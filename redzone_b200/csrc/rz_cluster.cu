@@ -70,7 +70,7 @@ __global__ void redzone_cluster_kernel(const ClusterParams p) {
     if (p.validate) {
         // Every CTA reads the same status word written by the validation kernels, so the
         // decision is uniform over the cluster and no CTA is left waiting at a barrier.
-        if (threadIdx.x == 0) s_abort = (__ldcg(p.status) & (ST_DUPLICATE | ST_RANGE)) != 0;
+        if (threadIdx.x == 0) s_abort = (__ldcg(p.status) & ST_INVALID) != 0;
         __syncthreads();
         if (s_abort) return;
     }

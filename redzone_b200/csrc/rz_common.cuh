@@ -20,6 +20,8 @@ enum : uint32_t {
     ST_TIMEOUT = 1u << 2,
     ST_INCONSISTENT = 1u << 3,  // orphan counts disagree (only possible with invalid input)
     ST_CAPACITY = 1u << 4,      // a produced list outgrew its capacity (nothing was moved)
+    ST_REFUSED = 1u << 5,       // another bit was set before a call that must not start then (set beside it)
+    ST_INVALID = ST_DUPLICATE | ST_RANGE | ST_REFUSED,  // a checked removal moves nothing
 };
 
 // 32-byte payload (u64 key + three u64 words in the streaming table; 8 x u32 otherwise).

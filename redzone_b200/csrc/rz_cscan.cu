@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(MAXB, 1) redzone_cscan_kernel(const CscanParam
         }
     }
 
-    if (threadIdx.x == 0) s_abort = p.validate ? ((__ldcg(p.status) & (ST_DUPLICATE | ST_RANGE)) != 0) : 0;
+    if (threadIdx.x == 0) s_abort = p.validate ? ((__ldcg(p.status) & ST_INVALID) != 0) : 0;
 
     // ---- this CTA's tile: index and tail item (needed only by the final moves) ----------------
     uint32_t rr[IPT];

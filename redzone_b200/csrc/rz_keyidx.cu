@@ -97,11 +97,15 @@ __global__ void ix_find_kernel(const unsigned long long* keys, const uint32_t* r
 
 // Rows and slots of the keys to delete (kNoRow when absent); every row is claimed (seen: one bit per
 // row of the list, zero before). A missing key, or one whose row is past the list, is an entry
-// outside it (ST_RANGE); a key given twice, or two keys that lead to one row, a duplicate.
+// outside it (ST_RANGE); a key given twice, or two keys that lead to one row, a duplicate. An earlier
+// call's error that is still in the status word refuses the call (ST_REFUSED): the index update goes by
+// the whole word, so the removal must not go by a part of it.
 __global__ void ix_claim_kernel(const unsigned long long* keys, const uint32_t* rows, uint32_t* seen, uint32_t mask,
                                 const unsigned long long* q, uint32_t count, uint32_t n, uint32_t* out_rows,
                                 uint32_t* out_slots, uint32_t* status) {
     pdl_begin();
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (__ldcg(status) & ~(ST_DUPLICATE | ST_RANGE)) != 0u)
+        atomicOr(status, ST_REFUSED);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const unsigned long long key = q[i];
         const uint32_t s = key >= kErasedKey ? kNoRow : find_slot(keys, mask, key);

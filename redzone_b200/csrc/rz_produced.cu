@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kProducedBlock, 1) redzone_produced_kernel(con
 
     if (threadIdx.x == 0) {
         s_R = 0;
-        s_abort = p.validate ? ((__ldcg(p.status) & (ST_DUPLICATE | ST_RANGE)) != 0) : 0;
+        s_abort = p.validate ? ((__ldcg(p.status) & ST_INVALID) != 0) : 0;
     }
     uint32_t rr[IPT];
     T src[IPT];

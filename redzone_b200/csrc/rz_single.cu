@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) validate_zero_kernel(uint32_t* __restrict
     pdl_begin();
     const uint32_t quads = words / 4, first = blockIdx.x * 1024u + threadIdx.x;
     uint4* q = reinterpret_cast<uint4*>(seen);
-    const bool mark = red && (ld_l2(status) & (ST_DUPLICATE | ST_RANGE)) == 0u;
+    const bool mark = red && (ld_l2(status) & ST_INVALID) == 0u;
     if (mark && (blockIdx.x + 1u) * 4096u > cut / 32u) {
         uint4 v[4];
 #pragma unroll

@@ -91,7 +91,7 @@ __device__ __forceinline__ void redzone_single_body(const SingleParams& p) {
 
     if (threadIdx.x == 0) {
         s_tag = (G > 1) ? ld_acquire(p.epoch) + 1u : 0u;
-        s_abort = p.validate ? ((__ldcg(p.status) & (ST_DUPLICATE | ST_RANGE)) != 0) : 0;
+        s_abort = p.validate ? ((__ldcg(p.status) & ST_INVALID) != 0) : 0;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && p.dev_len) *p.dev_len = (unsigned long long)(n - k);
 

@@ -183,3 +183,32 @@ def test_remove_by_key_follows_the_rule_under_every_flag(flag, k):
     assert np.array_equal(ix.find(dev_keys(keys_of(exp[: n - k]))).cpu().numpy(), np.arange(n - k))
     ix.close()
     c.close()
+
+
+@pytest.mark.parametrize("k", [2, 3000, 9000, 140000, 600000])
+def test_remove_by_key_behind_an_unread_error(ctx, k):
+    """A produced list over its capacity, removed without RZ_SYNC, leaves its error in the context: the
+    delete-by-key behind it returns that error and changes neither table nor index, on every schedule,
+    and the next one is exact."""
+    n, words = 4 * k + 1, 2
+    host = make_table(n, words, seed=k)
+    d = torch.from_numpy(host.view(np.int32).copy()).to(DEV)
+    ix = rz.KeyIndex(ctx, 2 * n)
+    ix.build(d)
+    pick = np.random.default_rng(k).choice(n, size=k, replace=False)
+    other = torch.zeros((64, 1), dtype=torch.int32, device=DEV)
+    p = rz.Producer(ctx, capacity=3)
+    p.reset(64)
+    p.produce_where_less(other, 1)
+    p.remove(other, flags=0)
+    with pytest.raises(rz.RedzoneError) as e:
+        ix.remove_by_key(d, n, dev_keys(keys_of(host)[pick]))
+    assert e.value.code == _native.RZ_ERR_NO_MEMORY
+    assert np.array_equal(d.cpu().numpy().view(np.uint32).reshape(n, words), host)
+    assert np.array_equal(ix.find(dev_keys(keys_of(host))).cpu().numpy(), np.arange(n))
+    assert ix.remove_by_key(d, n, dev_keys(keys_of(host)[pick])) == n - k
+    exp = host.copy()
+    oracle.remove(exp, pick.astype(np.uint32))
+    assert np.array_equal(d.cpu().numpy().view(np.uint32).reshape(n, words)[: n - k], exp[: n - k])
+    assert np.array_equal(ix.find(dev_keys(keys_of(exp[: n - k]))).cpu().numpy(), np.arange(n - k))
+    ix.close()
