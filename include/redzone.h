@@ -509,6 +509,14 @@ int rz_test_scatter(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, c
  * the device status word (bit 2 = timeout). The context's barrier state is reset afterwards.
  */
 int rz_test_barrier_timeout(rz_ctx* ctx, uint32_t spin_limit, uint32_t* status_bits);
+/*
+ * Failure check for calls of several kernels: of the launches that follow a kernel of the same call which
+ * left marks in the context's scratch (RZ_VALIDATE's second kernel, the grid kernel, the bulk
+ * schedule's and the partition's later ones), the one that comes after `after` others reports an error
+ * instead of being made (negative: none). The call returns RZ_ERR_CUDA, and the next one starts from
+ * clean scratch. Nothing fails on the GPU.
+ */
+int rz_test_fail_launch(rz_ctx* ctx, int32_t after);
 
 #ifdef __cplusplus
 }

@@ -563,8 +563,11 @@ int launch_bulk(rz_ctx* ctx, void* data, uint32_t n, const uint32_t* idx, uint32
     p.tpc = (ntiles + g - 1) / g;
     p.G = (ntiles + p.tpc - 1) / p.tpc;
     RZ_CUDA_TRY(ctx, launch_pdl(bulk_mark_kernel, 2 * ctx->sms, kBulkBlock, 0, s, p));
+    RZ_CUDA_TRY(ctx, injected_failure(ctx));
     RZ_CUDA_TRY(ctx, launch_pdl(bulk_split_kernel, p.G, kSplitBlock, smem_split, s, p));
+    RZ_CUDA_TRY(ctx, injected_failure(ctx));
     RZ_CUDA_TRY(ctx, launch_pdl(bulk_pair_kernel, 2 * ctx->sms, kSplitBlock, smem_split, s, p));
+    RZ_CUDA_TRY(ctx, injected_failure(ctx));
     RZ_CUDA_TRY(ctx, launch_pdl(bulk_fill_kernel, std::min<uint32_t>(p.nb, ctx->sms), kBulkBlock, smem_fill, s, p));
     return RZ_OK;
 }

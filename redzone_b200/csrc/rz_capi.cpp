@@ -227,6 +227,8 @@ static int remove_cfg(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes,
     if (k == 0 || k == n) {
         // Nothing moves (reference: redzone.hxx:651, Redzone_CPU.hxx handles it implicitly).
         if ((flags & RZ_VALIDATE) && !(flags & kPrevalidated) && k > 0) {
+            st = reset_if_dirty(ctx, s);
+            if (st != RZ_OK) return st;
             st = launch_validate(ctx, uint32_t(n), d_idx, uint32_t(k), s);
             if (st != RZ_OK) return st;
             ctx->last_kernels = 2;
@@ -540,6 +542,13 @@ int rz_test_scatter(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, c
     cudaSetDevice(ctx->device);
     return test_scatter(ctx, d_data, uint32_t(n), elem_bytes, d_pos, uint32_t(count),
                         reinterpret_cast<cudaStream_t>(stream));
+}
+
+int rz_test_fail_launch(rz_ctx* ctx, int32_t after) {
+    if (!ctx) return RZ_ERR_INVALID_ARG;
+    std::lock_guard<std::recursive_mutex> g(ctx->mu);
+    ctx->fail_launch = after < 0 ? -1 : after;
+    return RZ_OK;
 }
 
 int rz_test_barrier_timeout(rz_ctx* ctx, uint32_t spin_limit, uint32_t* status_bits) {

@@ -63,7 +63,7 @@ struct Workspace {
     unsigned long long* h_report = nullptr;  // pinned: {report number << 32 | status, number << 32 | length}
     unsigned long long* d_report = nullptr;  // the same words' device address
     bool stamps_on = false;
-    bool dirty = false;
+    bool dirty = false;              // to be zeroed before the next call (reset_if_dirty)
 };
 
 }  // namespace rz
@@ -84,6 +84,7 @@ struct rz_ctx {
     size_t scratch_held = 0;     // bytes of grown context scratch
     size_t scratch_limit = ~size_t(0);  // rz_set_scratch_limit: growth beyond it -> RZ_ERR_NO_MEMORY
     uint32_t report_seq = 0;             // number of the last report asked for (queue_status)
+    int fail_launch = -1;                // rz_test_fail_launch: launches until one fails; -1 for none
 };
 
 namespace rz {
@@ -104,6 +105,20 @@ int ensure_partition(rz_ctx* ctx, size_t n, size_t ntiles);
 // memory, or the stream is being captured): the caller then uses the grid schedule.
 int ensure_bulk(rz_ctx* ctx, size_t k, cudaStream_t s);
 int reset_if_dirty(rz_ctx* ctx, cudaStream_t s);
+// Call f, which launches kernels that leave marks in the context's scratch for the next of them: if one
+// of the launches fails, the scratch is zeroed before the next call.
+template <typename F>
+int launch_marking(rz_ctx* ctx, F f) {
+    const bool was = ctx->ws.dirty;
+    ctx->ws.dirty = true;
+    const int st = f();
+    if (st == RZ_OK) ctx->ws.dirty = was;
+    return st;
+}
+// What a launch that rz_test_fail_launch names returns in its place.
+inline cudaError_t injected_failure(rz_ctx* ctx) {
+    return ctx->fail_launch >= 0 && ctx->fail_launch-- == 0 ? cudaErrorLaunchFailure : cudaSuccess;
+}
 
 // Kernel launchers (rz_single.cu).
 struct LaunchInfo {

@@ -474,17 +474,8 @@ static MoveWsFn move_ws_fn(int w, size_t* smem) {
     }
 }
 
-int launch_partition(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* idx, uint32_t k,
-                     uint32_t flags, cudaStream_t s, LaunchInfo* info) {
-    const int items = part_items(int(w));
-    const uint32_t tile = uint32_t(kPartBlock * items);  // == kTileBytes / w for every width
-    const uint32_t ntiles = (n + tile - 1) / tile;
-    // The bit map is padded to whole tiles: the pipelined move copies a tile's words in one piece.
-    int st = ensure_partition(ctx, size_t(ntiles) * tile, ntiles);
-    if (st != RZ_OK) return st;
-    st = reset_if_dirty(ctx, s);
-    if (st != RZ_OK) return st;
-    const bool validate = (flags & RZ_VALIDATE) != 0;
+static int launch_tiles(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* idx, uint32_t k, int items,
+                        uint32_t ntiles, bool validate, cudaStream_t s, LaunchInfo* info) {
     // Scratch layout in tile_state: the ticket on its own 128-byte line, then staged and offset as
     // 32-bit arrays of ntiles rounded up to a multiple of 4, the tiles' and the runs' 16-byte records,
     // and the runs' totals.
@@ -510,9 +501,11 @@ int launch_partition(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint
                        : w == 8 ? partition_count_kernel<kTileBytes / 8 / 32>
                        : w == 16 ? partition_count_kernel<kTileBytes / 16 / 32>
                                  : partition_count_kernel<kTileBytes / 32 / 32>;
+    RZ_CUDA_TRY(ctx, injected_failure(ctx));
     RZ_CUDA_TRY(ctx, launch_pdl(count, cgrid, 256, 0, s, bits, n, ntiles, run, sc));
     const uint64_t dev_bit = 1ull << (ctx->device & 63);  // function attributes belong to a device (first 64)
     int grid = int(ntiles), block = kPartBlock;
+    RZ_CUDA_TRY(ctx, injected_failure(ctx));
     if ((reinterpret_cast<uintptr_t>(data) & 15u) == 0 && !ctx->ws.stamps_on) {
         size_t smem = 0;
         MoveWsFn f = move_ws_fn(int(w), &smem);
@@ -540,6 +533,20 @@ int launch_partition(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint
         info->launches += 3;  // mark, count, move
     }
     return RZ_OK;
+}
+
+int launch_partition(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* idx, uint32_t k,
+                     uint32_t flags, cudaStream_t s, LaunchInfo* info) {
+    const int items = part_items(int(w));
+    const uint32_t tile = uint32_t(kPartBlock * items);  // == kTileBytes / w for every width
+    const uint32_t ntiles = (n + tile - 1) / tile;
+    // The bit map is padded to whole tiles: the pipelined move copies a tile's words in one piece.
+    int st = ensure_partition(ctx, size_t(ntiles) * tile, ntiles);
+    if (st != RZ_OK) return st;
+    st = reset_if_dirty(ctx, s);
+    if (st != RZ_OK) return st;
+    const bool validate = (flags & RZ_VALIDATE) != 0;
+    return launch_marking(ctx, [&] { return launch_tiles(ctx, data, n, w, idx, k, items, ntiles, validate, s, info); });
 }
 
 }  // namespace rz

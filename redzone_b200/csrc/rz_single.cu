@@ -259,29 +259,26 @@ int launch_validate(rz_ctx* ctx, uint32_t n, const uint32_t* idx, uint32_t k, cu
     int st = ensure_seen(ctx, n);
     if (st != RZ_OK) return st;
     const uint64_t most = uint64_t(ctx->sms) * kValidateBlocksPerSm, blocks = (uint64_t(k) + 255) / 256;
-    RZ_CUDA_TRY(ctx, launch_pdl(blocks <= most ? validate_mark_kernel<1> : validate_mark_kernel<8>,
-                                uint32_t(std::max<uint64_t>(1, std::min(blocks, most))), 256, 0, s, idx, k, n, ctx->ws.seen,
-                                ctx->ws.status));
-    if (validate_marks(n, k)) {
-        const uint32_t words = uint32_t((uint64_t(n) + 31) / 32);
-        RZ_CUDA_TRY(ctx, launch_pdl(validate_zero_kernel, words / 4096 + 1, 256, 0, s, ctx->ws.seen, words, n - k, red,
+    return launch_marking(ctx, [&]() -> int {
+        RZ_CUDA_TRY(ctx, launch_pdl(blocks <= most ? validate_mark_kernel<1> : validate_mark_kernel<8>,
+                                    uint32_t(std::max<uint64_t>(1, std::min(blocks, most))), 256, 0, s, idx, k, n, ctx->ws.seen,
                                     ctx->ws.status));
-    } else {
-        const uint32_t grid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(ctx->sms) * 4, blocks)));
-        RZ_CUDA_TRY(ctx, launch_pdl(validate_clear_kernel, grid, 256, 0, s, idx, k, n, ctx->ws.seen));
-    }
-    return RZ_OK;
+        RZ_CUDA_TRY(ctx, injected_failure(ctx));
+        if (validate_marks(n, k)) {
+            const uint32_t words = uint32_t((uint64_t(n) + 31) / 32);
+            RZ_CUDA_TRY(ctx, launch_pdl(validate_zero_kernel, words / 4096 + 1, 256, 0, s, ctx->ws.seen, words, n - k, red,
+                                        ctx->ws.status));
+        } else {
+            const uint32_t grid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(ctx->sms) * 4, blocks)));
+            RZ_CUDA_TRY(ctx, launch_pdl(validate_clear_kernel, grid, 256, 0, s, idx, k, n, ctx->ws.seen));
+        }
+        return RZ_OK;
+    });
 }
 
-int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* idx, uint32_t k,
-                   const rz_launch_cfg& cfg_in, uint32_t flags, cudaStream_t s, LaunchInfo* info) {
-    rz_launch_cfg cfg = cfg_in;
-    int st = clamp_cfg(ctx, k, w, &cfg);
-    if (st != RZ_OK) return st;
-    st = ensure_lists(ctx, k);
-    if (st != RZ_OK) return st;
-    st = reset_if_dirty(ctx, s);
-    if (st != RZ_OK) return st;
+static int launch_scheduled(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* idx, uint32_t k,
+                            const rz_launch_cfg& cfg, uint32_t flags, cudaStream_t s, LaunchInfo* info) {
+    int st = RZ_OK;
     const bool validate = (flags & RZ_VALIDATE) != 0;
     int launches = 0;
     int sched = cfg.schedule;
@@ -420,6 +417,7 @@ int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
     attr[0].val.cooperative = grid > 1 ? 1 : 0;
     lc.attrs = attr;
     lc.numAttrs = 1;
+    RZ_CUDA_TRY(ctx, injected_failure(ctx));
     RZ_CUDA_TRY(ctx, cudaLaunchKernelEx(&lc, f, p));
     launches += 1;
     if (bulk) {
@@ -434,6 +432,18 @@ int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32
         info->launches = launches;
     }
     return RZ_OK;
+}
+
+int launch_redzone(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* idx, uint32_t k,
+                   const rz_launch_cfg& cfg_in, uint32_t flags, cudaStream_t s, LaunchInfo* info) {
+    rz_launch_cfg cfg = cfg_in;
+    int st = clamp_cfg(ctx, k, w, &cfg);
+    if (st != RZ_OK) return st;
+    st = ensure_lists(ctx, k);
+    if (st != RZ_OK) return st;
+    st = reset_if_dirty(ctx, s);
+    if (st != RZ_OK) return st;
+    return launch_marking(ctx, [&] { return launch_scheduled(ctx, data, n, w, idx, k, cfg, flags, s, info); });
 }
 
 // The end of a synchronous call (queue_status, rz_capi.cpp).

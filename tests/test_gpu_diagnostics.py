@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 import torch
 
+import oracle
 import redzone_b200 as rz
 from redzone_b200 import _native, workloads
 
@@ -56,3 +57,46 @@ def test_thrust_comparator_is_the_stable_remove(ctx):
         oracle.stable_remove(exp, idx)
         assert new_len == n - k
         assert np.array_equal(a.cpu().numpy().view(np.uint32)[: n - k], exp[: n - k])
+
+
+@pytest.mark.parametrize("route", ["validated", "validated_short", "all_removed", "bulk", "bulk_validated", "partition"])
+def test_scratch_is_clean_after_a_launch_that_failed(route):
+    """A launch that fails between the kernels of one call (reported by the library in its place) gives
+    RZ_ERR_CUDA, and the next call on the context, with another list, is the oracle's, on that route and on
+    the others."""
+    n, words = 2100001, 1
+    k = {"validated": 600001, "validated_short": 5000, "all_removed": n}.get(route, 100003)
+    c = rz.Context(0)
+    rng = np.random.default_rng(k)
+    host = rng.integers(0, 1 << 32, size=(n, words), dtype=np.uint64).astype(np.uint32)
+    bulk = rz.LaunchCfg(256, 4, 4, 0, 7)
+
+    def call(idx):
+        d = torch.from_numpy(host.view(np.int32).copy()).cuda()
+        i = torch.from_numpy(idx.view(np.int32).copy()).cuda()
+        if route == "partition":
+            c.partition(d, i, flags=rz.RZ_SYNC)
+            exp = np.delete(host, idx.astype(np.int64), axis=0)
+        else:
+            if route.startswith("bulk"):
+                c.remove_cfg(d, i, bulk, flags=rz.RZ_SYNC | (rz.RZ_VALIDATE if route == "bulk_validated" else 0))
+            else:
+                c.remove(d, i, flags=rz.RZ_SYNC | rz.RZ_VALIDATE)
+            exp = host.copy()
+            oracle.remove(exp, idx)
+        m = n - idx.size
+        assert np.array_equal(d.cpu().numpy().view(np.uint32)[:m], exp[:m])
+
+    launches = {"validated": 2, "validated_short": 1, "all_removed": 1, "bulk": 4, "bulk_validated": 5, "partition": 2}
+    for after in range(launches[route]):
+        assert rz._native.lib.rz_test_fail_launch(c.handle, after) == 0
+        with pytest.raises(rz.RedzoneError) as e:
+            call(rng.permutation(n)[:k].astype(np.uint32))
+        assert e.value.code == rz._native.RZ_ERR_CUDA
+        call(rng.permutation(n)[:k].astype(np.uint32))
+        d = torch.zeros((n, words), dtype=torch.int32, device="cuda")
+        tail = torch.arange(n - 700001, n, dtype=torch.int32, device="cuda")
+        assert c.remove(d, tail, flags=rz.RZ_SYNC | rz.RZ_VALIDATE) == n - 700001
+    rz._native.lib.rz_test_fail_launch(c.handle, -1)
+    call(rng.permutation(n)[:k].astype(np.uint32))
+    c.close()
