@@ -8,9 +8,10 @@
 // Grouping them by region is no help while a warp's stores still go to 32 different 128-byte lines
 // (2^24 int32 stores into 1 GiB: 760 us in random order, 560 grouped by 4 MB, 455 by 16 KB); stores
 // that share lines inside the warp instruction take 250-265 us (grouped by 1 KB, or sorted). So:
-//   sample: whether the holes crowd (a list with most of its removals in the tail, or in one part).
-//          Their stores meet in L2, so the grid kernel, which is launched next, does such a list. A word
-//          (gate) makes either it or the four kernels behind it return at once;
+//   sample: whether the holes crowd (a list with most of its removals in the tail, or in one part), or
+//          neighbours in the list lie near each other (sorted lists, runs in order). Their stores meet in
+//          L2, so the grid kernel, which is launched next, does such a list. A word (gate) makes
+//          either it or the four kernels behind it return at once;
 //   mark:  the V map (tail positions whose item is removed; phase A's red-zone bits) and the P map
 //          (entries that are no hole), and the number of holes in each of up to 2048 equal ranges of
 //          the list (buckets); the last block turns the counts into bucket offsets;
@@ -164,25 +165,54 @@ __device__ __forceinline__ bool last_block(uint32_t* done) {
     return s_last != 0u;
 }
 
-// Whether the list's holes crowd, from a sample of its entries: three eighths of them red or more, or an
-// eighth or more of them in one of 32 equal ranges (uniform lists: 64 of 2048 in each). One block, bound
-// by the latency of its loads: 4.8 us alone.
-constexpr uint32_t kCrowdSamples = 2 * kBulkBlock, kCrowdRanges = 32;
+// Whether the grid kernel stores the list's holes well, from 64 rows of 32 consecutive entries (its warps'
+// stores). Either the holes crowd: three eighths of the entries red or more, or an eighth or more of them
+// in one of 32 equal ranges (uniform lists: 64 of 2048 in each). Or a row's holes lie together: two points
+// for an entry with one of the next 8 within 1 KB of it, three more if one is in the same sector. Two
+// points per entry and more are the grid kernel's (grid / bulk us, points per entry; k = 2^24 of 2^28 and
+// 3 * 2^22 of 2^27): sorted 341 / 465 and 209 / 333 (2.6), sorted blocks of 8 in any order 429 / 458 and
+// 282 / 324 (2.3), runs of 2 427 / 433 and 297 / 309 (2.5), of 3 325 / 412 and 253 / 304 (3.3), of 256
+// 166 / 325 and 135 / 272 (4.8), four sorted lists in turn 324 / 444 and 214 / 334 (2.4); not so sorted blocks
+// of 4 483 / 462 and 335 / 324 (2.0), of 2 583 / 471 and 409 / 329 (1.3), sorted with half the entries
+// shuffled 621 / 475 and 418 / 338 (1.3). One block, bound by the latency of its loads.
+constexpr uint32_t kCrowdSamples = 2 * kBulkBlock, kCrowdRanges = 32, kCrowdAhead = 8;
 __global__ void __launch_bounds__(kBulkBlock) bulk_sample_kernel(const uint32_t* idx, uint32_t k, uint32_t cut, uint32_t* gate) {
-    __shared__ uint32_t s_in[kCrowdRanges + 1];
-    if (threadIdx.x <= kCrowdRanges) s_in[threadIdx.x] = 0u;
+    __shared__ uint32_t s_in[kCrowdRanges + 2];  // entries per range, red ones, points
+    if (threadIdx.x < kCrowdRanges + 2) s_in[threadIdx.x] = 0u;
     const float scale = float(kCrowdRanges) / float(cut);
+    const uint32_t lane = threadIdx.x & 31u, span = min(255u, cut >> 12);  // in short lists all entries are near
     pdl_begin();
     uint32_t r[2];
+    bool in[2];
 #pragma unroll
-    for (uint32_t j = 0; j < 2; ++j) r[j] = ld_l2(&idx[uint64_t(k) * (j * kBulkBlock + threadIdx.x) / kCrowdSamples]);
+    for (uint32_t j = 0; j < 2; ++j) {
+        const uint64_t row = (uint64_t(k) + 31u) / 32u * (j * (kBulkBlock / 32) + threadIdx.x / 32) / (kCrowdSamples / 32);
+        const uint64_t i = row * 32u + lane;
+        in[j] = i < k;
+        r[j] = in[j] ? ld_l2(&idx[i]) : 0u;
+    }
     __syncthreads();
+    uint32_t points = 0;
 #pragma unroll
-    for (uint32_t j = 0; j < 2; ++j)
-        atomicAdd(&s_in[r[j] < cut ? min(uint32_t(float(r[j]) * scale), kCrowdRanges - 1u) : kCrowdRanges], 1u);
+    for (uint32_t j = 0; j < 2; ++j) {
+        if (in[j]) atomicAdd(&s_in[r[j] < cut ? min(uint32_t(float(r[j]) * scale), kCrowdRanges - 1u) : kCrowdRanges], 1u);
+        bool near = false, same = false;
+#pragma unroll
+        for (uint32_t d = 1; d <= kCrowdAhead; ++d) {
+            const uint32_t o = __shfl_down_sync(0xffffffffu, r[j], d);
+            const bool there = __shfl_down_sync(0xffffffffu, uint32_t(in[j]), d) != 0u && lane + d < 32u;
+            near |= there && max(o, r[j]) - min(o, r[j]) <= span;
+            same |= there && (o >> 3) == (r[j] >> 3);
+        }
+        if (in[j]) points += (near ? 2u : 0u) + (same && near ? 3u : 0u);
+    }
+    points = __reduce_add_sync(0xffffffffu, points);
+    if (lane == 0u) atomicAdd(&s_in[kCrowdRanges + 1], points);
     __syncthreads();
-    const uint32_t c = threadIdx.x <= kCrowdRanges ? s_in[threadIdx.x] : 0u;
-    const bool crowd = __syncthreads_or(c >= kCrowdSamples / 8u * (threadIdx.x < kCrowdRanges ? 1u : 3u));
+    const uint32_t c = threadIdx.x <= kCrowdRanges + 1 ? s_in[threadIdx.x] : 0u;
+    const uint32_t most = threadIdx.x < kCrowdRanges ? kCrowdSamples / 8u
+                          : threadIdx.x == kCrowdRanges ? kCrowdSamples / 8u * 3u : kCrowdSamples * 2u;
+    const bool crowd = __syncthreads_or(c >= most);
     if (threadIdx.x == 0) *gate = crowd ? 1u : 0u;
 }
 
