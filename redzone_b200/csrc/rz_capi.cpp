@@ -75,9 +75,11 @@ int ensure_lists(rz_ctx* ctx, size_t k) {
     return RZ_OK;
 }
 
-int ensure_bulk(rz_ctx* ctx, size_t k, cudaStream_t s) {
+// Sized for whatever the orphan lists have room for, so that it grows only after they have grown: a
+// captured call keeps the addresses of both. (ensure_lists has run.)
+int ensure_bulk(rz_ctx* ctx, cudaStream_t s) {
     Workspace& ws = ctx->ws;
-    const size_t ctr = bulk_counter_words(), words = (k + 31) / 32;
+    const size_t ctr = bulk_counter_words(), k = ws.list_cap, words = (k + 31) / 32;
     if (ws.bulk_ctr && words <= ws.bulk_pmap_words && k <= ws.bulk_pairs_cap) return RZ_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {

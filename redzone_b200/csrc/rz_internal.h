@@ -103,7 +103,7 @@ int ensure_seen(rz_ctx* ctx, size_t n);
 int ensure_partition(rz_ctx* ctx, size_t n, size_t ntiles);
 // RZ_ERR_UNSUPPORTED when the bulk schedule's scratch is missing and cannot be had now (scratch limit, no
 // memory, or the stream is being captured): the caller then uses the grid schedule.
-int ensure_bulk(rz_ctx* ctx, size_t k, cudaStream_t s);
+int ensure_bulk(rz_ctx* ctx, cudaStream_t s);
 int reset_if_dirty(rz_ctx* ctx, cudaStream_t s);
 // Call f, which launches kernels that leave marks in the context's scratch for the next of them: if one
 // of the launches fails, the scratch is zeroed before the next call.

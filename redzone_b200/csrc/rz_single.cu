@@ -330,7 +330,7 @@ static int launch_scheduled(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, con
     if (sched == RZ_SCHED_BULK) {
         // The phase stamps are the grid kernel's.
         if (w == 4 && n > k && !ctx->ws.stamps_on) {
-            st = ensure_bulk(ctx, k, s);
+            st = ensure_bulk(ctx, s);
             if (st != RZ_OK && st != RZ_ERR_UNSUPPORTED) return st;
             bulk = st == RZ_OK;
         }

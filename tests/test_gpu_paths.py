@@ -462,3 +462,36 @@ def test_default_route_of_long_lists_by_their_order(ctx, order):
     assert us[0] < (1.2 if order != "random" else 0.85) * us[1], us
     del start, d, idx, out
     torch.cuda.empty_cache()
+
+
+def test_bulk_scratch_grows_with_the_lists_only():
+    """A context whose orphan lists have room for k removals takes the bulk schedule's scratch for k at its
+    first bulk call: later calls up to k leave it where it is, so a captured call stays right."""
+    c = rz.Context(0)
+    n, k0, k1 = 3000001, 200003, 20011
+    rng = np.random.default_rng(8)
+    wide = torch.zeros((n, 2), dtype=torch.int32, device=DEV)
+    c.remove_cfg(wide, on_gpu(rng.permutation(n)[:k0].astype(np.uint32)), rz.LaunchCfg(256, 4, 4, 0, 3), flags=rz.RZ_SYNC)
+    host = payload(n, 1, seed=8)
+    lists = {k: rng.permutation(n)[:k].astype(np.uint32) for k in (k1, k0)}
+    exps = {}
+    for k, idx in lists.items():
+        exps[k] = host.copy()
+        oracle.remove(exps[k], idx)
+    start, d, d_idx = on_gpu(host), on_gpu(host), on_gpu(lists[k1])
+    c.remove_cfg(d, d_idx, BULK, flags=rz.RZ_SYNC)
+    held = c.scratch_bytes
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        d.copy_(start)
+        c.remove_cfg(d, d_idx, BULK)
+    assert c.last_launch()[0] == 6
+    e = start.clone()
+    c.remove_cfg(e, on_gpu(lists[k0]), BULK, flags=rz.RZ_SYNC)
+    assert c.last_launch()[0] == 6 and c.scratch_bytes == held
+    assert np.array_equal(e.cpu().numpy().view(np.uint32)[: n - k0], exps[k0][: n - k0])
+    graph.replay()
+    assert c.sync_status() == 0
+    assert np.array_equal(d.cpu().numpy().view(np.uint32)[: n - k1], exps[k1][: n - k1])
+    c.close()
