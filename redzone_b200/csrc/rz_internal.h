@@ -59,6 +59,7 @@ struct Workspace {
     size_t bulk_pmap_words = 0;
     uint2* bulk_pairs = nullptr;     // bulk schedule: k (hole, item) pairs by bucket
     size_t bulk_pairs_cap = 0;
+    uint32_t bulk_wait = 0;          // calls before memory for it is asked for again
     unsigned long long* stamps = nullptr;     // optional phase timestamps, 8 per CTA
     unsigned long long* h_report = nullptr;  // pinned: {report number << 32 | status, number << 32 | length}
     unsigned long long* d_report = nullptr;  // the same words' device address
