@@ -28,8 +28,13 @@ constexpr int kPartBlock = 512;
 
 // Bound by the map's atomics (1.75e11 per second): kPartMarkLoads entries in flight per thread, and no
 // result asked for unless the list is validated. 10M entries of n = 100M: 58 us, 89 with one entry at
-// a time and the old word always asked for.
+// a time and the old word always asked for. Longer validated lists are marked by a kernel of its own in the
+// stream: blocks that start beside the last call's move kernel keep its split of the SM (nearly all
+// shared memory), and atomics that return a word then run at 0.7e11 per second instead of 1.1e11 (a call, us,
+// beside / behind, 4-byte items: 2^23 of 2^24 147 / 101, 10^7 of 10^8 282 / 216, 2^20 of 2^24 48 / 42, 2^18
+// 36.5 / 35.9, 1000 of 2^20 10.9 / 12.8). Marks without a result do not suffer from it.
 constexpr int kPartMarkLoads = 8;
+constexpr uint32_t kPartMarkBehind = 1u << 18;  // validated lists from here: not beside the kernel ahead
 template <bool VALIDATE>
 __global__ void __launch_bounds__(256) partition_mark_kernel(const uint32_t* __restrict__ idx, uint32_t k, uint32_t n,
                                                              uint32_t* __restrict__ bits, uint32_t* status) {
@@ -489,8 +494,13 @@ static int launch_tiles(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const u
     sc.run_total = reinterpret_cast<uint32_t*>(sc.run_recs + kPartMaxRuns);
     const uint32_t tag = 1u;
     const int mgrid = int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(ctx->sms) * 8, (uint64_t(k) + 255) / 256)));
-    RZ_CUDA_TRY(ctx, launch_pdl(validate ? partition_mark_kernel<true> : partition_mark_kernel<false>, uint32_t(mgrid), 256, 0,
-                                s, idx, k, n, ctx->ws.part_bits, ctx->ws.status));
+    if (validate && k >= kPartMarkBehind) {
+        partition_mark_kernel<true><<<mgrid, 256, 0, s>>>(idx, k, n, ctx->ws.part_bits, ctx->ws.status);
+        RZ_CUDA_TRY(ctx, cudaGetLastError());
+    } else {
+        RZ_CUDA_TRY(ctx, launch_pdl(validate ? partition_mark_kernel<true> : partition_mark_kernel<false>, uint32_t(mgrid),
+                                    256, 0, s, idx, k, n, ctx->ws.part_bits, ctx->ws.status));
+    }
     // Runs of 8 tiles (one per warp) or more, about four blocks per SM; kPartMaxRun * kPartMaxRuns tiles
     // are more than any list has (n < 2^32 items of 32 bytes: 2^22 tiles).
     const uint32_t most = std::max<uint32_t>(uint32_t(ctx->sms) * 4, (ntiles + kPartMaxRun - 1) / kPartMaxRun);
