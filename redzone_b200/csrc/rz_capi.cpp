@@ -463,9 +463,9 @@ int rz_keep(rz_ctx* ctx, void* d_data, int64_t n, uint32_t elem_bytes, const uin
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     st = grow(ctx, ctx->ws.keep_stage, ctx->ws.keep_cap, (size_t(m) * elem_bytes + 15) / 16 + 1, false);
     if (st != RZ_OK) return st;
+    ctx->last_kernels = 0;
     st = launch_keep(ctx, d_data, uint32_t(n), elem_bytes, d_keep, uint32_t(m), ctx->ws.keep_stage, s);
     if (st != RZ_OK) return st;
-    ctx->last_kernels = m > 0 ? 2 : 0;
     if (flags & RZ_SYNC) return read_status(ctx, s);
     return RZ_OK;
 }

@@ -171,7 +171,7 @@ void config_space(rz_launch_cfg* out);
 // red: nullable; the red-zone bitmap, which is marked too if the list is valid and validate_marks(n, k).
 bool validate_marks(uint32_t n, uint32_t k);
 int launch_validate(rz_ctx* ctx, uint32_t n, const uint32_t* idx, uint32_t k, cudaStream_t s, uint32_t* red = nullptr);
-// rz_keep: data[0..m) = old data[keep[j]] in two kernels; `stage` holds m items (those kept from [0, m)).
+// rz_keep: data[0..m) = old data[keep[j]]; `stage` holds m items.
 int launch_keep(rz_ctx* ctx, void* data, uint32_t n, uint32_t w, const uint32_t* keep, uint32_t m, void* stage,
                 cudaStream_t s);
 // Largest block size the single-list kernel for (w, items) can launch with.
