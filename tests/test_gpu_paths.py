@@ -624,3 +624,38 @@ def test_keep_of_all_items_without_order(ctx):
         us.append(best)
     assert ctx.sync_status() == 0
     assert us[0] < 2.3 * us[1], us
+
+
+def test_validation_of_a_tail_clears_a_big_map_by_entry(ctx):
+    """1.1M validated removals from the last tenth of 2^28 int32 (a map of 32 MB, cleared entry by entry) and of 32
+    items less (zeroed as a whole, a fifth longer): the oracle's result, a list with a duplicate refused in
+    between, and the longer list takes less time."""
+    k = (1 << 20) + (1 << 17)
+    us = []
+    g = torch.Generator(device=DEV).manual_seed(3)
+    for n in (1 << 28, (1 << 28) - 32):
+        d = torch.arange(n, dtype=torch.int32, device=DEV).view(-1, 1)
+        idx = (n - 1 - torch.randperm(n // 10, device=DEV, generator=g)[:k]).to(torch.int32)
+        bad = idx.clone()
+        bad[5] = bad[6]
+        for _ in range(2):
+            with pytest.raises(rz.RedzoneError) as e:
+                ctx.remove(d, bad, flags=rz.RZ_VALIDATE | rz.RZ_SYNC)
+            assert e.value.code == 2
+        want = d.clone()
+        ctx.remove_cfg(want, idx, rz.LaunchCfg(1024, 4, 2, 0, 3), flags=rz.RZ_SYNC)
+        ctx.remove(d, idx, flags=rz.RZ_VALIDATE | rz.RZ_SYNC)
+        assert torch.equal(d[: n - k], want[: n - k])
+        best = 1e9
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(10):
+                ctx.remove(d, idx, flags=rz.RZ_VALIDATE)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        us.append(best)
+        del d, want, idx, bad
+    torch.cuda.empty_cache()
+    assert us[0] < 0.95 * us[1], us
