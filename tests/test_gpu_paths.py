@@ -659,3 +659,63 @@ def test_validation_of_a_tail_clears_a_big_map_by_entry(ctx):
         del d, want, idx, bad
     torch.cuda.empty_cache()
     assert us[0] < 0.95 * us[1], us
+
+
+@pytest.mark.parametrize("shift", [0, 4])
+@pytest.mark.parametrize("n,k", [(40, 39), (5000, 300), (9001, 4000), (70000, 9000), (600001, 70000), (600001, 200003),
+                                 (1600008, 200001), (1600007, 200001)])
+def test_32_byte_items_on_and_off_whole_sectors(ctx, n, k, shift):
+    """32-byte items in a list on 32 bytes (whole-sector stores, or halves in dense lists) and 16 bytes off (always
+    two stores): every schedule, a validated call, keep, partition, a produced list and a batch; dense and
+    sparse around n = 8 k."""
+    rng = np.random.default_rng(n + k)
+    host = payload(n, 8, seed=k)
+    idx = rng.permutation(n)[:k].astype(np.uint32)
+    exp = host.copy()
+    oracle.remove(exp, idx)
+    d_idx, start = on_gpu(idx), on_gpu(host).reshape(-1)
+    room = torch.zeros(n * 8 + 8, dtype=torch.int32, device=DEV)
+    d = room[shift: shift + n * 8].view(n, 8)
+
+    def check(call, want=exp[: n - k]):
+        room.fill_(7)
+        d.copy_(start.view(n, 8))
+        call()
+        got = d[: want.shape[0]].cpu().numpy().view(np.uint32)
+        assert np.array_equal(got, want)
+        edge = torch.cat([room[:shift], room[shift + n * 8:]])
+        assert (edge == 7).all()
+
+    check(lambda: ctx.remove(d, d_idx, flags=rz.RZ_SYNC))
+    check(lambda: ctx.remove(d, d_idx, flags=rz.RZ_SYNC | rz.RZ_VALIDATE))
+    for sched in (1, 2, 3, 4, 5, 6, 7):
+        if sched == 1 and k > 20000:
+            continue
+        for items in (1, 4):
+            check(lambda: ctx.remove_cfg(d, d_idx, rz.LaunchCfg(256, items, 2, 0, sched), flags=rz.RZ_SYNC))
+    check(lambda: ctx.partition(d, d_idx, flags=rz.RZ_SYNC), np.delete(host, idx.astype(np.int64), axis=0))
+    check(lambda: ctx.keep(d, d_idx, flags=rz.RZ_SYNC), host[idx])
+    if k <= 1 << 18:
+        keys = np.full(n, 900, np.uint32)
+        keys[idx] = 1
+        p = rz.Producer(ctx, capacity=k)
+        d_keys = on_gpu(keys)
+
+        def produced():
+            p.reset(n)
+            p.produce_where_less(d_keys, 500)
+            p.remove(d, flags=rz.RZ_SYNC)
+
+        room.fill_(7)
+        d.copy_(start.view(n, 8))
+        produced()
+        want = host.copy()
+        oracle.remove(want, p.download()[0])
+        assert np.array_equal(d[: n - k].cpu().numpy().view(np.uint32), want[: n - k])
+    room.fill_(7)
+    d.copy_(start.view(n, 8))
+    plan = rz.BatchPlan(ctx, [(d, d_idx)])
+    plan.launch()
+    torch.cuda.synchronize()
+    plan.close()
+    assert np.array_equal(d[: n - k].cpu().numpy().view(np.uint32), exp[: n - k])
