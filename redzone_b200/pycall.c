@@ -14,13 +14,47 @@ typedef int (*list_fn)(void*, void*, int64_t, uint32_t, const uint32_t*, int64_t
 static PyObject *s_shape, *s_data_ptr, *s_numel, *s_element_size;
 static PyObject *get_device, *get_stream;  // torch's current device and its raw current stream
 
+// A whole number: an int, or what says that it is one (a numpy integer).
+static int whole(PyObject* v, unsigned long long* out) {
+    PyObject* i = PyLong_Check(v) ? Py_NewRef(v) : PyNumber_Index(v);
+    if (!i) return -1;
+    *out = PyLong_AsUnsignedLongLong(i);
+    Py_DECREF(i);
+    return PyErr_Occurred() ? -1 : 0;
+}
+
 // An integer-valued method of a tensor.
 static int ask(PyObject* t, PyObject* method, unsigned long long* out) {
     PyObject* v = PyObject_CallMethodNoArgs(t, method);
     if (!v) return -1;
-    *out = PyLong_AsUnsignedLongLong(v);
+    const int bad = whole(v, out);
     Py_DECREF(v);
-    return PyErr_Occurred() ? -1 : 0;
+    return bad;
+}
+
+// Items of a tensor, and elements per item. Its shape is a tuple, or with other owners of device memory any
+// sequence.
+static int sizes(PyObject* t, unsigned long long* n, unsigned long long* per) {
+    PyObject* shape = PyObject_GetAttr(t, s_shape);
+    if (!shape) return -1;
+    PyObject* dims = PySequence_Fast(shape, "a shape is a sequence");
+    Py_DECREF(shape);
+    if (!dims) return -1;
+    const Py_ssize_t axes = PySequence_Fast_GET_SIZE(dims);
+    int bad = 0;
+    if (axes < 1) {
+        PyErr_SetString(PyExc_IndexError, "the list needs a first axis");
+        bad = -1;
+    }
+    *per = 1;
+    for (Py_ssize_t i = 0; i < axes && !bad; ++i) {
+        unsigned long long d = 0;
+        bad = whole(PySequence_Fast_GET_ITEM(dims, i), &d);
+        if (i == 0) *n = d;
+        else *per *= d;
+    }
+    Py_DECREF(dims);
+    return bad;
 }
 
 static int address(PyObject* v, void** out) {
@@ -35,25 +69,16 @@ static PyObject* call(PyObject* self, PyObject* const* a, Py_ssize_t nargs) {
     if (nargs != 6) return PyErr_Format(PyExc_TypeError, "call takes 6 arguments");
     void *fn, *ctx, *stream = NULL;
     if (address(a[0], &fn) || address(a[1], &ctx)) return NULL;
-    unsigned long long data, idx, k, elem;
-    PyObject* shape = PyObject_GetAttr(a[2], s_shape);
-    if (!shape) return NULL;
-    if (!PyTuple_Check(shape) || PyTuple_GET_SIZE(shape) < 1) {
-        Py_DECREF(shape);
-        return PyErr_Format(PyExc_IndexError, "the list needs a first axis");
-    }
-    const long long n = PyLong_AsLongLong(PyTuple_GET_ITEM(shape, 0));
-    unsigned long long per = 1;
-    for (Py_ssize_t i = 1; i < PyTuple_GET_SIZE(shape); ++i) per *= (unsigned long long)PyLong_AsLongLong(PyTuple_GET_ITEM(shape, i));
-    Py_DECREF(shape);
-    if (PyErr_Occurred() || ask(a[2], s_element_size, &elem) || ask(a[2], s_data_ptr, &data) || ask(a[3], s_data_ptr, &idx) ||
-        ask(a[3], s_numel, &k))
+    unsigned long long n = 0, per = 1, data, idx, k, elem;
+    if (sizes(a[2], &n, &per) || ask(a[2], s_element_size, &elem) || ask(a[2], s_data_ptr, &data) ||
+        ask(a[3], s_data_ptr, &idx) || ask(a[3], s_numel, &k))
         return NULL;
     const uint32_t flags = (uint32_t)PyLong_AsUnsignedLongMask(a[4]);
     if (PyErr_Occurred()) return NULL;
     if (a[5] != Py_None) {
         if (address(a[5], &stream)) return NULL;
     } else {
+        if (!get_stream) return PyErr_Format(PyExc_RuntimeError, "no current stream before bind");
         PyObject* dev = PyObject_CallNoArgs(get_device);
         PyObject* raw = dev ? PyObject_CallOneArg(get_stream, dev) : NULL;
         Py_XDECREF(dev);
@@ -65,7 +90,7 @@ static PyObject* call(PyObject* self, PyObject* const* a, Py_ssize_t nargs) {
     int64_t new_len = 0;
     int st;
     Py_BEGIN_ALLOW_THREADS
-    st = ((list_fn)fn)(ctx, (void*)(uintptr_t)data, n, (uint32_t)(per * elem), (const uint32_t*)(uintptr_t)idx, (int64_t)k,
+    st = ((list_fn)fn)(ctx, (void*)(uintptr_t)data, (int64_t)n, (uint32_t)(per * elem), (const uint32_t*)(uintptr_t)idx, (int64_t)k,
                        &new_len, flags, stream);
     Py_END_ALLOW_THREADS
     return PyLong_FromLongLong(st ? -(long long)st : (long long)new_len);

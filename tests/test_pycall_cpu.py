@@ -1,7 +1,10 @@
 """The Python extension behind Context's list calls (redzone_b200/pycall.c), with a callback in the
 place of the library's functions: what it passes, what it returns, what it refuses."""
 import ctypes
+import subprocess
+import sys
 
+import numpy as np
 import pytest
 import torch
 
@@ -53,3 +56,46 @@ def test_list_call_looks_the_stream_up_and_refuses_what_has_no_sizes():
     with pytest.raises(TypeError):
         rzcall.call(addr, 0, data, idx, 0)
     assert len(seen) == 1
+
+
+class Buffer:
+    """Device memory of another owner: what Context's list calls ask of a tensor, and no more."""
+
+    def __init__(self, shape, numel, itemsize=4, at=0x1000):
+        self.shape, self._numel, self._itemsize, self._at = shape, numel, itemsize, at
+
+    def data_ptr(self):
+        return self._at
+
+    def element_size(self):
+        return self._itemsize
+
+    def numel(self):
+        return self._numel
+
+
+@pytest.mark.parametrize("shape", [[7, 2], np.array([7, 2]), (np.int64(7), 2), torch.Size([7, 2])])
+def test_list_call_takes_any_sequence_and_integer(shape):
+    seen = []
+
+    @FN
+    def fn(ctx, data, n, elem, idx, k, new_len, flags, stream):
+        seen.append((data, n, elem, idx, k))
+        new_len[0] = n - k
+        return 0
+
+    addr = ctypes.cast(fn, ctypes.c_void_p).value
+    got = rzcall.call(addr, 1, Buffer(shape, 14), Buffer([3], np.int64(3), at=0x2000), 0, 1)
+    assert got == 4 and seen == [(0x1000, 7, 8, 0x2000, 3)]
+    for bad, error in ((Buffer([], 0), IndexError), (Buffer([2.5, 2], 5), TypeError), (Buffer(7, 7), TypeError)):
+        with pytest.raises(error):
+            rzcall.call(addr, 1, bad, Buffer([3], 3), 0, 1)
+    assert len(seen) == 1
+
+
+def test_list_call_without_a_bound_stream_is_an_error():
+    code = ("import torch\nfrom redzone_b200 import _native\nm = _native.load_pycall()\n"
+            "t = torch.zeros(4, dtype=torch.int32)\n"
+            "try:\n    m.call(1, 1, t, t, 0, None)\nexcept RuntimeError as e:\n    print('refused', e)\n")
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=_native.PKG.parent)
+    assert out.returncode == 0 and "refused" in out.stdout, out
