@@ -8,6 +8,7 @@ import ctypes
 import importlib.machinery
 import importlib.util
 import re
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -193,8 +194,9 @@ _sig("rz_phase_stamps", c_i32, [c_vp, c_i32])
 _sig("rz_read_phase_stamps", c_i32, [c_vp, ctypes.POINTER(c_u64), c_i32, ctypes.POINTER(c_i32)])
 
 
-# The list calls (pycall.c): None when the extension was built for another interpreter or not at all.
-PYCALL_PATH = PKG / "_lib" / "_rzcall.so"
+# The list calls (pycall.c): None when the extension was not built, or for another interpreter only (its name
+# carries the binary interface, as an installed extension's does).
+PYCALL_PATH = PKG / "_lib" / ("_rzcall" + sysconfig.get_config_var("EXT_SUFFIX"))
 LIST_CALLS = {name: ctypes.cast(getattr(lib, name), c_vp).value
               for name in ("rz_remove", "rz_remove_host_idx", "rz_partition", "rz_keep")}
 

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import concurrent.futures as cf
 import os
+import shutil
 import subprocess
 import sys
 import sysconfig
@@ -21,7 +22,7 @@ OUT_DIR = PKG / "_lib"
 OBJ_DIR = PKG / "_lib" / "obj"
 LIB = OUT_DIR / "libredzone_b200.so"
 E2E = OUT_DIR / "rz_e2e"
-PYCALL = OUT_DIR / "_rzcall.so"
+PYCALL = OUT_DIR / ("_rzcall" + sysconfig.get_config_var("EXT_SUFFIX"))  # of this interpreter's binary interface
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -85,9 +86,9 @@ def build(verbose: bool = False, quiet: bool = False) -> Path:
 
 def build_pycall(quiet: bool = False) -> Path | None:
     """The Python extension behind Context's list calls (redzone_b200/pycall.c). Without Python's
-    headers it is left out, and those calls go through ctypes."""
+    headers or a C compiler it is left out, and those calls go through ctypes."""
     src, include = PKG / "pycall.c", Path(sysconfig.get_paths()["include"])
-    if not (include / "Python.h").exists():
+    if not (include / "Python.h").exists() or not shutil.which("gcc"):
         return None
     if PYCALL.exists() and PYCALL.stat().st_mtime >= src.stat().st_mtime:
         return PYCALL

@@ -1,6 +1,7 @@
 """The Python extension behind Context's list calls (redzone_b200/pycall.c), with a callback in the
 place of the library's functions: what it passes, what it returns, what it refuses."""
 import ctypes
+import importlib.machinery
 import subprocess
 import sys
 
@@ -99,3 +100,16 @@ def test_list_call_without_a_bound_stream_is_an_error():
             "try:\n    m.call(1, 1, t, t, 0, None)\nexcept RuntimeError as e:\n    print('refused', e)\n")
     out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=_native.PKG.parent)
     assert out.returncode == 0 and "refused" in out.stdout, out
+
+
+def test_extension_is_named_for_its_interpreter_and_left_out_without_a_compiler(monkeypatch, tmp_path):
+    """Another Python does not find this one's extension (a name without its binary interface would load
+    there), and a build without a C compiler goes on without it."""
+    from redzone_b200 import build
+    assert build.PYCALL == _native.PYCALL_PATH
+    assert build.PYCALL.name == "_rzcall" + importlib.machinery.EXTENSION_SUFFIXES[0] != "_rzcall.so"
+    monkeypatch.setattr(build, "PYCALL", tmp_path / build.PYCALL.name)
+    monkeypatch.setenv("PATH", str(tmp_path))
+    assert build.build_pycall(quiet=True) is None
+    monkeypatch.setattr(_native, "PYCALL_PATH", tmp_path / "_rzcall.cpython-300-x86_64-linux-gnu.so")
+    assert _native.load_pycall() is None
