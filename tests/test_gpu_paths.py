@@ -719,3 +719,28 @@ def test_32_byte_items_on_and_off_whole_sectors(ctx, n, k, shift):
     torch.cuda.synchronize()
     plan.close()
     assert np.array_equal(d[: n - k].cpu().numpy().view(np.uint32), exp[: n - k])
+
+
+@pytest.mark.parametrize("n,k,dense", [(1 << 24, 1 << 21, 3), (50000017, 1 << 24, 0), (50000017, (1 << 24) - 5, 2)])
+def test_bulk_schedule_beyond_one_tile(ctx, n, k, dense):
+    """Buckets of several fill tiles (holes three times as dense in a 32nd of the list, which the sample does not
+    call crowded) and blocks with more than one tile of orphans to pair (a third of the list removed), against
+    the grid schedule."""
+    g = torch.Generator(device=DEV).manual_seed(k)
+    idx = torch.randperm(n, device=DEV, generator=g)
+    if dense:
+        lo, hi = n // 4, n // 4 + n // 32
+        inside = (idx >= lo) & (idx < hi)
+        share = min(dense * (k / n), 0.95)
+        many = idx[inside][: int(share * (hi - lo))]
+        idx = torch.cat([many, idx[~inside][: k - many.numel()]])
+        idx = idx[torch.randperm(idx.numel(), device=DEV, generator=g)]
+    idx = idx[:k].to(torch.int32)
+    start = torch.arange(n, dtype=torch.int32, device=DEV).view(-1, 1)
+    a, b = start.clone(), start
+    ctx.remove_cfg(a, idx, BULK, flags=rz.RZ_SYNC)
+    assert ctx.last_launch()[0] == 6
+    ctx.remove_cfg(b, idx, rz.LaunchCfg(1024, 4, 2, 0, 3), flags=rz.RZ_SYNC)
+    assert torch.equal(a[: n - k], b[: n - k])
+    del idx, start, a, b
+    torch.cuda.empty_cache()
