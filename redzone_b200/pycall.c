@@ -16,11 +16,15 @@ static PyObject *get_device, *get_stream;  // torch's current device and its raw
 
 // A whole number: an int, or what says that it is one (a numpy integer).
 static int whole(PyObject* v, unsigned long long* out) {
-    PyObject* i = PyLong_Check(v) ? Py_NewRef(v) : PyNumber_Index(v);
-    if (!i) return -1;
-    *out = PyLong_AsUnsignedLongLong(i);
-    Py_DECREF(i);
-    return PyErr_Occurred() ? -1 : 0;
+    if (PyLong_CheckExact(v)) {
+        *out = PyLong_AsUnsignedLongLong(v);
+    } else {
+        PyObject* i = PyNumber_Index(v);
+        if (!i) return -1;
+        *out = PyLong_AsUnsignedLongLong(i);
+        Py_DECREF(i);
+    }
+    return *out == (unsigned long long)-1 && PyErr_Occurred() ? -1 : 0;
 }
 
 // An integer-valued method of a tensor.
@@ -35,23 +39,26 @@ static int ask(PyObject* t, PyObject* method, unsigned long long* out) {
 // Items of a tensor, and elements per item. Its shape is a tuple, or with other owners of device memory any
 // sequence.
 static int sizes(PyObject* t, unsigned long long* n, unsigned long long* per) {
-    PyObject* shape = PyObject_GetAttr(t, s_shape);
-    if (!shape) return -1;
-    PyObject* dims = PySequence_Fast(shape, "a shape is a sequence");
-    Py_DECREF(shape);
+    PyObject* dims = PyObject_GetAttr(t, s_shape);
+    if (dims && !PyTuple_Check(dims)) {
+        PyObject* tuple = PySequence_Tuple(dims);
+        Py_DECREF(dims);
+        dims = tuple;
+    }
     if (!dims) return -1;
-    const Py_ssize_t axes = PySequence_Fast_GET_SIZE(dims);
+    const Py_ssize_t axes = PyTuple_GET_SIZE(dims);
     int bad = 0;
     if (axes < 1) {
         PyErr_SetString(PyExc_IndexError, "the list needs a first axis");
         bad = -1;
+    } else {
+        bad = whole(PyTuple_GET_ITEM(dims, 0), n);
     }
     *per = 1;
-    for (Py_ssize_t i = 0; i < axes && !bad; ++i) {
-        unsigned long long d = 0;
-        bad = whole(PySequence_Fast_GET_ITEM(dims, i), &d);
-        if (i == 0) *n = d;
-        else *per *= d;
+    for (Py_ssize_t i = 1; i < axes && !bad; ++i) {
+        unsigned long long d;
+        bad = whole(PyTuple_GET_ITEM(dims, i), &d);
+        if (!bad) *per *= d;
     }
     Py_DECREF(dims);
     return bad;
