@@ -575,13 +575,15 @@ def test_partition_validation_of_half_a_list_costs_less_than_the_rest(ctx):
 
 
 @pytest.mark.parametrize("words,shift", [(1, 0), (2, 0), (4, 0), (8, 0), (8, 4)])
-@pytest.mark.parametrize("share", ["wide", "edge", "next", "half", "most", "all"])
+@pytest.mark.parametrize("share", ["wide", "sparse", "edge", "next", "half", "most", "all"])
 def test_keep_of_long_lists(ctx, words, shift, share):
     """rz_keep in a list of 192 MiB, the first size with 64-byte loads, around 64 bytes per kept item where
-    they end and around seven eighths where all items are staged: any order, rows given twice, an entry past
-    the end, 32-byte items on and off 32 bytes."""
-    n = (192 << 20) // (4 * words)
-    m = {"wide": n // 1000, "edge": n * 4 * words // 64, "next": n * 4 * words // 64 + 1, "half": n // 2 + 1,
+    they end, at 2^20 items and a sixteenth (16-byte items: a 32nd) where they stay out of L1, and around
+    seven eighths where all items are staged: any order, rows given twice, an entry past the end, 32-byte
+    items on and off 32 bytes."""
+    n = ((544 if share == "sparse" else 192) << 20) // (4 * words)
+    m = {"wide": n // 1000, "sparse": n // (32 if words == 4 else 16), "edge": n * 4 * words // 64,
+         "next": n * 4 * words // 64 + 1, "half": n // 2 + 1,
          "most": n - n // 8, "all": n - n // 8 + 1}[share]
     if m > n:
         pytest.skip("more than there are")
