@@ -53,10 +53,10 @@ __global__ void redzone_single_kernel(const SingleParams p) {
 // the map cleared entry by entry; 65k entries with one: 8.4 us, with eight: 9.1).
 constexpr uint64_t kValidateBlocksPerSm = 8;
 // Lists of more than n / 256 entries: the map is zeroed as a whole (n / 8 bytes; n = 50M: 3 us)
-// instead of entry by entry (2M entries: 21 us). Maps of 32 MB and more: from n / 64 entries, since entries that
-// lie together are cleared in less than such a map (a call, us, whole / by entry; removals from the tail: 2^20 of
-// 2^28 62 / 51, 2^21 of 2^28 96 / 91, of 2^27 61 / 78; uniform: 2^20 of 2^28 89 / 90).
-constexpr uint32_t kValidateMapShare = 256, kValidateBigMapShare = 64, kValidateBigMap = 1u << 28;
+// instead of entry by entry (2M entries: 21 us). Maps over 16 MB: from n / 64 entries, since entries that lie
+// together are cleared in less than such a map (a call, us, whole / by entry; removals from the tail: 2^19 of 2^27
+// 33.5 / 34.5, 2^20 of 2^28 62 / 51, 2^21 of 2^28 96 / 91, of 2^27 61 / 78; uniform: 2^20 of 2^28 89 / 90).
+constexpr uint32_t kValidateMapShare = 256, kValidateBigMapShare = 64, kValidateBigMap = 1u << 27;
 template <int LOADS>
 __global__ void __launch_bounds__(256) validate_mark_kernel(const uint32_t* __restrict__ idx, uint32_t k, uint32_t n,
                                                             uint32_t* __restrict__ seen, uint32_t* status) {
@@ -256,7 +256,7 @@ int default_cfg(const rz_ctx* ctx, uint32_t n, uint32_t k, uint32_t w, rz_launch
 }
 
 bool validate_marks(uint32_t n, uint32_t k) {
-    return uint64_t(n) < uint64_t(n < kValidateBigMap ? kValidateMapShare : kValidateBigMapShare) * k;
+    return uint64_t(n) < uint64_t(n <= kValidateBigMap ? kValidateMapShare : kValidateBigMapShare) * k;
 }
 
 int launch_validate(rz_ctx* ctx, uint32_t n, const uint32_t* idx, uint32_t k, cudaStream_t s, uint32_t* red) {
