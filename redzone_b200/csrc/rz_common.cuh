@@ -275,8 +275,9 @@ __device__ __forceinline__ void tma_load_1d(void* dst_smem, const void* src, uin
 }
 
 // ---- programmatic dependent launch ----------------------------------------------------------------
-// Loads for kernels that may start before their inputs' writer has ended: through L2, never the
-// non-coherent path, whose lines may be older than the wait.
+// Kernels that may start before their inputs' writer has ended must not read them by the non-coherent path, whose
+// lines may be older than the wait (any other load after the wait sees what was written before it). The
+// compiler takes that path for loads through pointers that are const and __restrict__: these loads never do.
 __device__ __forceinline__ uint32_t ld_l2(const uint32_t* p) { return __ldcg(p); }
 __device__ __forceinline__ uint2 ld_l2(const uint2* p) { return __ldcg(p); }
 __device__ __forceinline__ uint4 ld_l2(const uint4* p) { return __ldcg(p); }

@@ -13,7 +13,7 @@
 // goes into the context's status word, which the removal (as after those passes) and the index
 // update look at before they change anything. So the whole call is queued at once and the host
 // waits for it once. Bound by the random accesses of the probes and by that wait: deleting 65521 of
-// 4.2M 32-byte records by key, inserting as many and looking as many up takes 97 us, and took 165 us
+// 4.2M 32-byte records by key, inserting as many and looking as many up takes 67 us, and took 155 us
 // with a wait after the lookup, validation passes over the rows, and 64-bit rows made from 32-bit ones
 // by the caller. (Keys and rows in one 16-byte slot made the calls 7 % faster but the build slower by
 // half: 134 MB of slots do not stay in L2.)
