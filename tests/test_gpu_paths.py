@@ -508,7 +508,13 @@ def test_bulk_schedule_without_memory_for_its_scratch():
     want = d.clone()
     c.remove_cfg(want, idx, rz.LaunchCfg(1024, 4, 2, 0, 3), flags=rz.RZ_SYNC)
     torch.cuda.synchronize()
-    taken = torch.empty(torch.cuda.mem_get_info()[0] - (96 << 20), dtype=torch.uint8, device=DEV)
+    taken = []
+    size = torch.cuda.mem_get_info()[0] - (96 << 20)
+    while size > 16 << 20 and torch.cuda.mem_get_info()[0] > 112 << 20:
+        try:
+            taken.append(torch.empty(min(size, torch.cuda.mem_get_info()[0] - (96 << 20)), dtype=torch.uint8, device=DEV))
+        except torch.OutOfMemoryError:
+            size //= 2
     try:
         cfg = rz.LaunchCfg(1024, 4, 2, 0, 7)
         c.remove_cfg(d, idx, cfg, flags=rz.RZ_SYNC)
